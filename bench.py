@@ -726,7 +726,7 @@ def run_frames(args) -> int:
     out = {}
     check = sorted({0, nf - 1})  # frames whose images are compared with the FP64 oracle
     imgs = {}
-    # fused: 0 no, 1 groups with frame pairs back-projected together, 2 groups only
+    # fused: 0 no, 1 groups (frame pairs of equal normalization counted), 2 groups
     arms = {"plain": ("f32", False, 0), "batched_f32": ("f32", True, 0), "batched": ("f16", True, 0),
             "fused_launch_only": ("f16", True, 2), "fused_f32": ("f32", True, 1), "fused": ("f16", True, 1)}
     for arm, (storage, batched, fused) in arms.items():

@@ -128,7 +128,7 @@ def segment_table(g: Geometry):
 
 
 def bp_staged_rows(g: Geometry) -> dict:
-    """The per-view back projector's staged-row buffer (gf_bp_staged_rows)."""
+    """The per-view back projector's staged-row buffer, one warp per column (gf_bp_staged_rows)."""
     lo, hi, rb = ctypes.c_int32(), ctypes.c_int32(), ctypes.c_int32()
     _ck(lib().gf_bp_staged_rows(ctypes.byref(g.c()), ctypes.byref(lo), ctypes.byref(hi), ctypes.byref(rb)))
     return {"pad_lo": lo.value, "pad_hi": hi.value, "rbuf": rb.value}
@@ -363,13 +363,13 @@ class Batch:
 
     def set_fused(self, fused: bool = True, pairs: bool = True) -> None:
         """Fused groups: frames that match (any subset counts) run each stage
-        as one launch; with pairs, frames of one subset count and equal
-        normalization back-project two per warp (gf_batch_set_fused 1, else 2;
+        as one launch; with pairs, groups() counts the frame pairs of one subset
+        count and equal normalization (gf_batch_set_fused 1, else 2;
         fused=False: 0)."""
         _ck(lib().gf_batch_set_fused(self.h, 0 if not fused else (1 if pairs else 2)))
 
     def groups(self) -> tuple:
-        """(units, largest group, frame pairs back-projected together) as the batch stands now."""
+        """(units, largest group, frame pairs of equal subset count and mask) as the batch stands now."""
         n, big, pr = ctypes.c_int32(), ctypes.c_int32(), ctypes.c_int32()
         _ck(lib().gf_batch_groups(self.h, ctypes.byref(n), ctypes.byref(big), ctypes.byref(pr)))
         return n.value, big.value, pr.value

@@ -6,9 +6,7 @@
 // and tile shapes form fused groups of up to kMaxFrames, whatever their
 // subset counts, whose sub-iterations run every stage as one launch over the
 // frames that have that subset (fused_subiteration); every other frame is a
-// unit of its own.  Frames of a group with the same subset count and equal
-// normalization masks (the frames of one scanner and normalization)
-// back-project two per warp, sharing the per-view geometry and the mask rows.
+// unit of its own.
 //
 // One iteration of every unit is captured once: a fork event on the batch's
 // origin stream, each unit's kernels on the stream of its first frame (a
@@ -32,10 +30,10 @@ using namespace gf;
 struct gf_batch {
   std::vector<gf_recon*> frames;
   int device = 0;
-  int fused = 0;  // gf_batch_set_fused: 0 off, 1 groups (paired back projection where masks match), 2 groups
+  int fused = 0;  // gf_batch_set_fused: 0 off, 1 or 2 groups (1: gf_batch_groups counts pairs of equal masks)
   std::vector<std::vector<int>> units;  // frame indices: a fused group, or one frame
-  // per unit and member: its pairing class (the first member with the same
-  // subset count and an equal normalization mask), or -1 (back-projected alone)
+  // per unit and member: its class (the first member with the same subset
+  // count and an equal normalization mask), or -1
   std::vector<std::vector<int>> cls;
   int* d_flag = nullptr;                // device flag of the mask comparison
   cudaStream_t origin = nullptr;
@@ -80,10 +78,9 @@ static void make_units(gf_batch* b) {
   }
 }
 
-// Which frames of a fused group may back-project two per warp: those with
-// the same subset count whose static normalization masks (every subset, in
-// that count's layout) are equal bit for bit, compared on the device after
-// the frames' queued work (their loads) has finished.
+// The frames of a fused group that have the same subset count and equal
+// normalization masks (every subset, in that count's layout), compared on the
+// device after the frames' queued work (their loads) has finished.
 static gf_status check_masks(gf_batch* b) {
   b->cls.assign(b->units.size(), {});
   for (size_t k = 0; k < b->units.size(); k++) {
@@ -98,11 +95,15 @@ static gf_status check_masks(gf_batch* b) {
         if (b->cls[k][i] != (int)i) continue;  // not a class leader
         const gf_recon* l = b->frames[u[i]];
         if (l->ctx->plan.nsub != r->ctx->plan.nsub) continue;
-        bool same = l->cal == r->cal;
-        if (!same) {
+        bool same = false;
+        {
           GF_CK(cudaStreamSynchronize(l->ctx->stream));
           GF_CK(cudaStreamSynchronize(r->ctx->stream));
-          GF_CK(launch_differs(l->cal, r->cal, (size_t)l->ctx->plan.all_elems(), b->d_flag, b->origin));
+          // the same geometry and subset count: the same form on both sides
+          const float* ml = l->cal ? l->cal : reinterpret_cast<const float*>(l->mask);
+          const float* mr = r->cal ? r->cal : reinterpret_cast<const float*>(r->mask);
+          const size_t n = l->cal ? (size_t)l->ctx->plan.all_elems() : l->mask_words();
+          GF_CK(launch_differs(ml, mr, n, b->d_flag, b->origin));
           int flag = 1;
           GF_CK(cudaMemcpyAsync(&flag, b->d_flag, sizeof(int), cudaMemcpyDeviceToHost, b->origin));
           GF_CK(cudaStreamSynchronize(b->origin));
@@ -131,14 +132,9 @@ static gf_status unit_iteration(gf_batch* b, size_t k) {
   for (int i : u) smax = std::max(smax, b->frames[i]->ctx->plan.nsub);
   for (int s = 0; s < smax; s++) {
     std::vector<gf_recon*> G;
-    std::vector<int> C;
-    for (size_t j = 0; j < u.size(); j++) {
-      gf_recon* r = b->frames[u[j]];
-      if (r->ctx->plan.nsub <= s) continue;
-      G.push_back(r);
-      C.push_back(b->cls[k][j]);
-    }
-    GF_TRY(fused_subiteration(G.data(), (int)G.size(), C.data(), st));
+    for (int i : u)
+      if (b->frames[i]->ctx->plan.nsub > s) G.push_back(b->frames[i]);
+    GF_TRY(fused_subiteration(G.data(), (int)G.size(), st));
   }
   return GF_OK;
 }
@@ -228,7 +224,6 @@ static gf_status capture(gf_batch* b) {
   make_units(b);
   // the frames' streams must be idle before they join the capture
   for (gf_recon* r : b->frames) GF_CK(cudaStreamSynchronize(r->ctx->stream));
-  GF_TRY(check_masks(b));
   std::vector<bool> prof(b->frames.size());
   std::vector<gf_ctx*> ctxs;  // each context once: frames may share one
   std::vector<int64_t> l0;
@@ -301,7 +296,6 @@ gf_status gf_batch_iterate(gf_batch* b, int32_t n, int32_t use_graph) {
   GF_CK(cudaSetDevice(b->device));
   if (!use_graph) {
     make_units(b);
-    GF_TRY(check_masks(b));
     for (int it = 0; it < n; it++) {
       for (size_t ku = 0; ku < b->units.size(); ku++) {
         const std::vector<int>& u = b->units[ku];

@@ -89,7 +89,12 @@ gf_status gf_ctx::ensure_scratch() {
   GF_TRY(alloc_t(p.nvoxp, &s_img2));
   GF_TRY(alloc_t(p.nvoxp, &s_numer));
   GF_TRY(alloc_t(p.nvoxp, &s_denom));
-  GF_TRY(alloc_t((size_t)p.amax * p.g.nrad * p.PS, &s_cc));
+  const size_t n = (size_t)p.amax * p.g.nrad * p.PS;
+  GF_TRY(alloc_t(n, &s_pairs));
+  if (bp_uses_tiles(p)) {
+    GF_TRY(alloc_t(n / 32, &s_mask));
+    GF_TRY(alloc_t(s_dirty_words() + 1, &s_dirty));
+  }
   return GF_OK;
 }
 
@@ -120,19 +125,15 @@ FpArgs gf_ctx::fp_args(int subset, const float* img_zfast) const {
   return a;
 }
 
-BpArgs gf_ctx::bp_args(int subset, const void* cc, float* numer, float* denom, int storage) const {
+BpArgs gf_ctx::bp_args(int subset, const BpFrame& f, int storage) const {
   BpArgs b{};
   b.g = dg;
   b.subset = subset;
   b.na = plan.sub_nang[subset];
   b.nfr = 1;
-  b.fr[0].corrcal = cc;
-  b.fr[0].numer = numer;
-  b.fr[0].denom = denom;
+  b.fr[0] = f;
   b.storage = storage;
   b.fast = bp_form == GF_BP_PER_VIEW ? 1 : 0;
-  b.pad_lo = bpp.pad_lo;
-  b.rbuf = bpp.rbuf;
   return b;
 }
 
@@ -258,7 +259,7 @@ gf_status gf_create(const gf_geometry* g, int32_t nsubsets, int32_t device, gf_c
     cudaGetLastError();
   }
   gf_ctx* c = new gf_ctx();
-  c->bpp = bp_fast_pads(plan);
+  c->bp_warps = bp_uses_tiles(plan) ? 8 : 4;
   c->plan = std::move(plan);
   c->fps = std::move(fps);
   c->device = device;
@@ -486,9 +487,29 @@ gf_status gf_back_project(gf_ctx* c, const float* d_corr, const float* d_calib, 
   if (!d_corr || !d_calib || !d_numer || !d_denom) return set_error(GF_ERR_ARG, "null buffer");
   GF_TRY(c->ensure_scratch());
   const int na = c->plan.sub_nang[subset];
-  GF_LAUNCH(c, launch_corrcal_from_file(c->dg, c->d_rowmap, subset, na, d_corr, d_calib, c->s_cc, c->stream));
-  BpArgs b = c->bp_args(subset, c->s_cc, c->s_numer, c->s_denom, 0);
-  GF_LAUNCH(c, launch_bp(b, c->bp_warps, c->stream));
+  if (!bp_uses_tiles(c->plan)) {
+    GF_LAUNCH(c, launch_pairs_from_file(c->dg, c->d_rowmap, subset, na, d_corr, d_calib, c->s_pairs, nullptr, c->stream));
+    const BpArgs b = c->bp_args(subset, BpFrame{c->s_pairs, nullptr, nullptr, c->s_numer, c->s_denom}, 0);
+    GF_LAUNCH(c, launch_bp(b, c->bp_tile(0), c->stream));
+  } else {
+    // the tiles, and one warp per column for a mask that they do not take:
+    // which of the two runs is known on the device only
+    const size_t nd = c->s_dirty_words();
+    int* general = reinterpret_cast<int*>(c->s_dirty + nd);
+    float* corr = reinterpret_cast<float*>(c->s_pairs);
+    GF_CK(cudaMemsetAsync(c->s_dirty, 0, (nd + 1) * sizeof(unsigned), c->stream));
+    GF_LAUNCH(c, launch_ratio_from_file(c->dg, c->d_rowmap, subset, na, d_corr, d_calib, corr, c->s_mask, c->s_dirty,
+                                        general, c->stream));
+    BpArgs b = c->bp_args(subset, BpFrame{corr, c->s_mask, c->s_dirty, c->s_numer, c->s_denom}, 0);
+    b.general = general;
+    GF_LAUNCH(c, launch_bp(b, c->bp_tile(0), c->stream));
+    GF_LAUNCH(c, launch_pairs_from_file(c->dg, c->d_rowmap, subset, na, d_corr, d_calib, c->s_pairs, general, c->stream));
+    b.fr[0] = BpFrame{c->s_pairs, nullptr, nullptr, c->s_numer, c->s_denom};
+    BpTile columns = c->bp_tile(0);
+    columns.zr = 0;
+    columns.warps = 4;
+    GF_LAUNCH(c, launch_bp(b, columns, c->stream));
+  }
   GF_LAUNCH(c, launch_zfast_to_file(c->dg, c->s_numer, 1.f, 0, d_numer, c->stream));
   GF_LAUNCH(c, launch_zfast_to_file(c->dg, c->s_denom, 1.f, 0, d_denom, c->stream));
   return GF_OK;

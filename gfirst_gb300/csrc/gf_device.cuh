@@ -38,6 +38,11 @@ template <> __device__ __forceinline__ float2 pair_from<float2>(float2 v) { retu
 template <> __device__ __forceinline__ __half2 pair_from<__half2>(float2 v) { return __float22half2_rn(v); }
 template <> __device__ __forceinline__ __nv_bfloat162 pair_from<__nv_bfloat162>(float2 v) { return __float22bfloat162_rn(v); }
 
+template <class T> __device__ __forceinline__ T elem_from(float v);
+template <> __device__ __forceinline__ float elem_from<float>(float v) { return v; }
+template <> __device__ __forceinline__ __half elem_from<__half>(float v) { return __float2half_rn(v); }
+template <> __device__ __forceinline__ __nv_bfloat16 elem_from<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
+
 __device__ __forceinline__ float lerp_rn(float a, float b, float w) { return __fmaf_rn(w, __fsub_rn(b, a), a); }
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return min(max(v, lo), hi); }
 // The update ratio of divVxVGPU (GFIRST_GPU_Kernels.cu:173-182): NUMER/DENOM,

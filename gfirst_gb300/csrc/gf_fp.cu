@@ -15,17 +15,17 @@
 //      interpolation whose integer offset and fraction are the same for all
 //      planes of a segment, so a thread walks a run of R consecutive planes
 //      with R+1 shared loads and R interpolations per step;
-//  (3) applies the ratio in the epilogue and writes (corr, calib) pairs
-//      contiguously in the radial-major layout the back projector reads.
+//  (3) applies the ratio in the epilogue and writes the ratios contiguously
+//      in the radial-major layout the back projector reads.
 // Work per ray-sample is one shared load and one 1-D interpolation instead of
 // eight texel reads; the image and data stream from HBM once.
 #include "gf_kernels.h"
 
 namespace gf {
 
-template <int R, bool RATIO, bool FULL, int STORE>
+// PAIRS: the ratio output is (ratio, mask) pairs.
+template <int R, bool RATIO, bool FULL, int STORE, bool PAIRS>
 __global__ void __launch_bounds__(512) fp_kernel(const FpArgs a) {
-  using Pair = typename PairT<STORE>::type;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int lc = a.lc, cw = a.cw;
   int4* offs = reinterpret_cast<int4*>(smraw);              // [lc]
@@ -120,7 +120,6 @@ __global__ void __launch_bounds__(512) fp_kernel(const FpArgs a) {
   if (run.x < 0 || !active) return;
   const DevSeg sg = g.seg[run.x];
   const size_t base = ((size_t)tl * g.nrad + ird) * g.PS;
-  const float2 sentinel = make_float2(-1000.f, -1000.f);
 #pragma unroll
   for (int j = 0; j < R; j++) {
     if (j < run.z) {
@@ -135,19 +134,27 @@ __global__ void __launch_bounds__(512) fp_kernel(const FpArgs a) {
         const float2 db = F.dbg[o];
         const float s = __fadd_rn(proj, db.y);
         const float corr = (s >= 0.01f) ? __fdiv_rn(db.x, s) : -1000.f;
-        Pair* cc_out = static_cast<Pair*>(F.corrcal);
-        const Pair cc = pair_from<Pair>(make_float2(corr, F.cal[o]));
-        cc_out[o] = cc;
-        if (j == 0 && (run.w & 1)) cc_out[o - 1] = (run.x == 0) ? cc : pair_from<Pair>(sentinel);
-        if (j == run.z - 1 && (run.w & 2)) cc_out[o + 1] = (run.x == 0) ? cc : pair_from<Pair>(sentinel);
+        auto put = [&](auto* out, auto v, auto sentinel) {
+          out[o] = v;
+          if (j == 0 && (run.w & 1)) out[o - 1] = (run.x == 0) ? v : sentinel;
+          if (j == run.z - 1 && (run.w & 2)) out[o + 1] = (run.x == 0) ? v : sentinel;
+        };
+        if constexpr (PAIRS) {
+          using P = typename PairT<STORE>::type;
+          put(static_cast<P*>(F.corr), pair_from<P>(make_float2(corr, F.cal[o])),
+              pair_from<P>(make_float2(-1000.f, -1000.f)));
+        } else {
+          using T = typename ElemT<STORE>::type;
+          put(static_cast<T*>(F.corr), elem_from<T>(corr), elem_from<T>(-1000.f));
+        }
       }
     }
   }
 }
 
-template <int R, bool RATIO, bool FULL, int STORE>
+template <int R, bool RATIO, bool FULL, int STORE, bool PAIRS>
 static cudaError_t launch_fp_t(const FpArgs& a, const FpSchedule& s, cudaStream_t st) {
-  auto k = fp_kernel<R, RATIO, FULL, STORE>;
+  auto k = fp_kernel<R, RATIO, FULL, STORE, PAIRS>;
   size_t smem = s.smem_bytes();
   cudaError_t e = allow_max_smem(k);
   if (e != cudaSuccess) return e;
@@ -158,16 +165,20 @@ static cudaError_t launch_fp_t(const FpArgs& a, const FpSchedule& s, cudaStream_
   return cudaGetLastError();
 }
 
-template <int R>
-static cudaError_t launch_fp_r(const FpArgs& a, const FpSchedule& s, cudaStream_t st) {
-  if (!a.fr[0].corrcal) return launch_fp_t<R, false, true, 0>(a, s, st);
+template <int R, bool PAIRS>
+static cudaError_t launch_fp_p(const FpArgs& a, const FpSchedule& s, cudaStream_t st) {
   switch (a.storage) {
-    case 0:
-      return a.fr[0].proj_full ? launch_fp_t<R, true, true, 0>(a, s, st) : launch_fp_t<R, true, false, 0>(a, s, st);
-    case 1: return launch_fp_t<R, true, false, 1>(a, s, st);
-    case 2: return launch_fp_t<R, true, false, 2>(a, s, st);
+    case 0: return launch_fp_t<R, true, false, 0, PAIRS>(a, s, st);
+    case 1: return launch_fp_t<R, true, false, 1, PAIRS>(a, s, st);
+    case 2: return launch_fp_t<R, true, false, 2, PAIRS>(a, s, st);
     default: return cudaErrorInvalidValue;
   }
+}
+
+template <int R>
+static cudaError_t launch_fp_r(const FpArgs& a, const FpSchedule& s, cudaStream_t st) {
+  if (!a.fr[0].corr) return launch_fp_t<R, false, true, 0, false>(a, s, st);
+  return a.fr[0].cal ? launch_fp_p<R, true>(a, s, st) : launch_fp_p<R, false>(a, s, st);
 }
 
 cudaError_t launch_fp(const FpArgs& a, const FpSchedule& s, cudaStream_t st) {
@@ -175,15 +186,15 @@ cudaError_t launch_fp(const FpArgs& a, const FpSchedule& s, cudaStream_t st) {
   // every frame of a launch has the outputs of frame 0 (one kernel variant)
   for (int f = 0; f < (a.nfr > 1 ? a.nfr : 1); f++) {
     const FpFrame& F = a.fr[f];
-    if (!F.img || (!F.corrcal && !F.proj_full)) return cudaErrorInvalidValue;
-    if (!F.corrcal != !a.fr[0].corrcal || !F.proj_full != !a.fr[0].proj_full) return cudaErrorInvalidValue;
-    if (F.corrcal && (!F.dbg || !F.cal)) return cudaErrorInvalidValue;
+    if (!F.img || (!F.corr && !F.proj_full)) return cudaErrorInvalidValue;
+    if (!F.corr != !a.fr[0].corr || !F.proj_full != !a.fr[0].proj_full) return cudaErrorInvalidValue;
+    if (F.corr && (!F.dbg || !F.cal != !a.fr[0].cal)) return cudaErrorInvalidValue;
     // the subset's angles: subset + l*nsub for l < na, all inside [0, nang)
     if (F.nsub < 1 || F.subset < 0 || F.subset >= F.nsub || F.na < 1 ||
         F.na != (a.g.nang - F.subset + F.nsub - 1) / F.nsub)
       return cudaErrorInvalidValue;
   }
-  if (a.fr[0].corrcal && a.fr[0].proj_full && a.storage != 0) return cudaErrorInvalidValue;
+  if (a.fr[0].corr && a.fr[0].proj_full) return cudaErrorInvalidValue;  // one output or the other
   switch (s.R) {
     case 9: return launch_fp_r<9>(a, s, st);
     case 17: return launch_fp_r<17>(a, s, st);

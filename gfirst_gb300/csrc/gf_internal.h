@@ -68,16 +68,20 @@ struct gf_ctx {
   // Bumped whenever a launch parameter that a captured graph holds changes
   // (the projectors' tile shapes, gf_tune); gf_batch recaptures on a change.
   int64_t gen = 0;
-  int bp_warps = 4;      // back-projector warps (columns) per block (eight blocks per SM fit the register cap)
+  int bp_warps = 4;      // back-projector warps (slice runs of one column tile) per block
   // back projector's axial interpolation for doubles images and the operator
   // entry point (gf_set_bp_form); triples images always use GF_BP_PER_VOXEL
   int bp_form = GF_BP_PER_VIEW;
-  gf::BpPads bpp;        // staged-row buffer of the per-view form
   float* s_img = nullptr;
   float* s_img2 = nullptr;
   float* s_numer = nullptr;
   float* s_denom = nullptr;
-  float2* s_cc = nullptr;
+  // gf_back_project: one subset as (ratio, mask) pairs, or as ratios with the
+  // mask's bits and dirty bits, then the general flag
+  float2* s_pairs = nullptr;
+  unsigned* s_mask = nullptr;
+  unsigned* s_dirty = nullptr;
+  size_t s_dirty_words() const { return (size_t)plan.amax * plan.g.nrad * ((plan.g.nseg + 31) / 32); }
 
   gf_status alloc(size_t bytes, void** p);
   template <class T> gf_status alloc_t(size_t n, T** p) {
@@ -86,7 +90,8 @@ struct gf_ctx {
   gf_status ensure_scratch();
   gf_status ensure_gtab(float sigma3d);
   gf::FpArgs fp_args(int subset, const float* img_zfast) const;
-  gf::BpArgs bp_args(int subset, const void* corrcal, float* numer, float* denom, int storage) const;
+  gf::BpArgs bp_args(int subset, const gf::BpFrame& f, int storage) const;
+  gf::BpTile bp_tile(int storage) const { return gf::bp_tile(plan, bp_warps, storage == GF_STORE_F32 ? 4 : 2); }
 };
 
 struct gf_recon {
@@ -101,9 +106,25 @@ struct gf_recon {
   float* psf = nullptr;
   float* ratio = nullptr;  // the back projector's update ratio NUMER/DENOM, z-fast
   float* filt = nullptr;
-  void* corrcal = nullptr;  // (ratio, mask) pairs of the current subset, gf_recon_params::storage
+  void* corr = nullptr;  // the current subset for the back projector, gf_recon_params::storage
   float2* dbg[2] = {nullptr, nullptr};
+  // normalization mask of every subset: values beside the ratios (one warp per
+  // column), or one bit per row with its dirty bits (column tiles)
   float* cal = nullptr;
+  unsigned* mask = nullptr;
+  unsigned* dirty = nullptr;
+  size_t mask_words() const { return (size_t)ctx->plan.all_elems() / 32; }
+  size_t dirty_words() const {
+    return (size_t)ctx->plan.g.nang * ctx->plan.g.nrad * ((ctx->plan.g.nseg + 31) / 32);
+  }
+  const float* cal_of(int s) const { return cal ? cal + ctx->plan.sub_off[s] : nullptr; }
+  // subset s for the back projector (the update ratio goes to `ratio`)
+  gf::BpFrame bp_frame(int s) const {
+    const gf::Plan& pl = ctx->plan;
+    const int64_t off = pl.sub_off[s];
+    if (cal) return gf::BpFrame{corr, nullptr, nullptr, ratio, nullptr};
+    return gf::BpFrame{corr, mask + off / 32, dirty + off / pl.PS * ((pl.g.nseg + 31) / 32), ratio, nullptr};
+  }
   float* proj_ref = nullptr;
   bool cyl_proj_ready = false;  // proj_ref holds the unit-cylinder projection (modes 1-3)
   float* proj_t = nullptr;  // triples projection, file layout (VLOR split weights)
@@ -167,7 +188,6 @@ bool fusable(const gf_recon* a, const gf_recon* b);
 // kMaxFrames frames, the back projection one launch per subset count among
 // them, on stream st (the group's: its first member's, which need not take
 // part in every step) with the first frame's tables.  Advances every frame's
-// cursor.  cls: frames with the same class >= 0 (same subset count and
-// normalization mask; per-view back projector) back-project two per warp.
-gf_status fused_subiteration(gf_recon* const* G, int nfr, const int* cls, cudaStream_t st);
+// cursor.
+gf_status fused_subiteration(gf_recon* const* G, int nfr, cudaStream_t st);
 }  // namespace gf

@@ -9,7 +9,13 @@
 
 namespace gf {
 
-// (ratio, mask) pair storage of the per-subset sinogram.
+// Storage of the per-subset sinogram that the back projector reads
+// (gf_recon_params::storage): ratios for the column tiles, (ratio, mask) pairs
+// for one warp per column.
+template <int S> struct ElemT;
+template <> struct ElemT<0> { using type = float; };
+template <> struct ElemT<1> { using type = __half; };
+template <> struct ElemT<2> { using type = __nv_bfloat16; };
 template <int S> struct PairT;
 template <> struct PairT<0> { using type = float2; };
 template <> struct PairT<1> { using type = __half2; };
@@ -29,9 +35,9 @@ constexpr int kMaxFrames = 16;
 // ---- forward projector (gf_fp.cu) ----
 struct FpFrame {
   const float* img;        // z-fast image (after the forward PSF)
-  const float2* dbg;       // subset layout (data*RES, max(bg*RES,0)); with corrcal
-  const float* cal;        // subset layout normalization mask; with corrcal
-  void* corrcal;           // subset layout (corr, calib) pairs output, or null
+  const float2* dbg;       // subset layout (data*RES, max(bg*RES,0)); with corr
+  const float* cal;        // subset layout mask: corr holds (ratio, mask) pairs; null: ratios
+  void* corr;              // subset layout output for the back projector, or null
   float* proj_full;        // file-layout projection output, or null
   int subset, nsub, na;    // the frame's subset, its subset count and the subset's angles
 };
@@ -39,7 +45,7 @@ struct FpArgs {
   DevGeom g;               // g.nsub unused: each frame names its own
   const int4* runs;        // FpSchedule::runs as (seg, p0, n, pad)
   int nruns, padl, cw, lc;
-  int storage;             // corrcal pair type: 0 float2, 1 __half2, 2 __nv_bfloat162
+  int storage;             // ratio element type: 0 float, 1 __half, 2 __nv_bfloat16
   int nfr;                 // frames in this launch (grid z); 0 is taken as 1
   FpFrame fr[kMaxFrames];
 };
@@ -47,7 +53,9 @@ cudaError_t launch_fp(const FpArgs& a, const FpSchedule& s, cudaStream_t st);
 
 // ---- back projector (gf_bp.cu) ----
 struct BpFrame {
-  const void* corrcal;     // subset layout (corr, calib) pairs
+  const void* in;          // subset layout: ratios (tiles) or (ratio, mask) pairs
+  const unsigned* mask;    // tiles: the mask, one bit per row (32 rows a word), 1 unmasked
+  const unsigned* dirty;   // tiles: per (angle, radial bin) a bit per segment, 1 where a row of it is masked
   float* numer;            // z-fast
   float* denom;            // z-fast
 };
@@ -55,21 +63,26 @@ struct BpFrame {
 struct BpArgs {
   DevGeom g;
   int subset, na;          // na: angles in this subset
-  int nfr;                 // frames in this launch (grid y); 0 is taken as 1
-  BpFrame fr[kMaxFrames];
-  int storage;             // corrcal pair type, as FpArgs::storage
+  int nfr;                 // frames in this launch
+  int storage;             // element type of BpFrame::in, as FpArgs::storage
   // Axial interpolation: 0 per voxel with the reference's rounding (the
-  // oracle's sums bit for bit), 1 per view (BpPads; within 1e-5 of it).
+  // oracle's sums bit for bit), 1 per view (within 1e-5 of it).
   int fast;
-  int pad_lo, rbuf;        // fast form: staged-row buffer per warp (BpPads)
   // 0: write the column sums to BpFrame::numer and ::denom; 1: write the
   // update ratio NUMER/DENOM (divVxVGPU) to ::numer alone (::denom unused).
   int ratio;
+  // device flag, or null: 1 where the mask holds other values than 1 and
+  // -1000; the tiles then end at once, and one warp per column where it is 0
+  const int* general;
+  // set by the launchers: words of a dirty entry, row stride of a bin
+  // (elements), mask words of a bin, bytes of a slot and of what precedes its
+  // rows (tiles); the staged-row buffer (BpPads)
+  int nsw, rs, mw, slot_bytes, rows_at;
+  int pad_lo, rbuf;
+  BpFrame fr[kMaxFrames];
 };
-cudaError_t launch_bp(const BpArgs& a, int warps, cudaStream_t st);
-// Per-view form over a.nfr = 2n frames as n pairs (frames 2p, 2p + 1) that
-// share their normalization mask: one warp per column and pair.
-cudaError_t launch_bp_pairs(const BpArgs& a, int warps, cudaStream_t st);
+cudaError_t launch_bp(const BpArgs& a, const BpTile& tile, cudaStream_t st);
+cudaError_t launch_bp_tiles(const BpArgs& a, const BpTile& tile, cudaStream_t st);  // gf_bp_tile.cu
 // Lets kernel k use up to the device's opt-in shared memory per block.  Every
 // call sets the same value, so host threads that launch one kernel with
 // different shared-memory sizes at the same time cannot undo each other's
@@ -130,11 +143,23 @@ cudaError_t launch_build_dbg(const DevGeom& g, const int2* rowmap, const float* 
                              cudaStream_t st);
 cudaError_t launch_build_cal(const DevGeom& g, const int2* rowmap, const float* proj_ref, const float* norm,
                              float* cal, cudaStream_t st);
-cudaError_t launch_corrcal_from_file(const DevGeom& g, const int2* rowmap, int subset, int na, const float* corr,
-                                     const float* calib, float2* corrcal, cudaStream_t st);
+// The normalization mask of every subset as bits (32 rows a word) and its
+// dirty bits (BpFrame::mask, ::dirty; dirty must hold 0 before).
+cudaError_t launch_build_mask(const DevGeom& g, const int2* rowmap, const float* proj_ref, const float* norm,
+                              unsigned* mask, unsigned* dirty, cudaStream_t st);
+// One subset from the file layout: its ratios with the mask's bits and dirty
+// bits, *general = 1 where a mask value is neither 1 nor -1000 (dirty and
+// general must hold 0 before); or (ratio, mask) pairs, where *general is set
+// (null: always).
+cudaError_t launch_ratio_from_file(const DevGeom& g, const int2* rowmap, int subset, int na, const float* corr,
+                                   const float* calib, float* out, unsigned* mask, unsigned* dirty, int* general,
+                                   cudaStream_t st);
+cudaError_t launch_pairs_from_file(const DevGeom& g, const int2* rowmap, int subset, int na, const float* corr,
+                                   const float* calib, float2* out, const int* general, cudaStream_t st);
+// cal: (ratio, mask) pairs; null: ratios
 cudaError_t launch_ratio_gather(const DevGeom& g, const int2* rowmap, int subset, int na, const float* proj_full,
-                                const float* datos_v, const float2* dbg_t, const float* cal, void* corrcal,
-                                int storage, cudaStream_t st);
+                                const float* datos_v, const float2* dbg_t, const float* cal, void* out, int storage,
+                                cudaStream_t st);
 cudaError_t launch_ratio_file(const DevGeom& g, int subset, const float* proj, const float* data, const float* bg,
                               float* corr, cudaStream_t st);
 cudaError_t launch_norm_mask(const DevGeom& g, const float* proj_blank, const float* blank, float* calib,

@@ -151,6 +151,58 @@ BpPads bp_fast_pads(const Plan& p) {
   return b;
 }
 
+// The tile shape of a plan, whether or not it is used.
+static BpTile tile_shape(const Plan& p, int warps, int elem_bytes) {
+  BpTile t;
+  t.warps = warps;
+  // Slices of a run: longer runs share the radial interpolation of a row and a
+  // view's set-up among more voxels, shorter ones waste less at the ends of a
+  // segment and make more CTAs.  12 / 16 slices, us a launch: 535 / 523 (128 x
+  // 128 x 159 voxels, 53 segments, 10 angles, per-view form), 701 / 705 (per
+  // voxel), 332 / 322 (15 segments, 21 angles), 201 / 226 (96^3), 102 / 116 (72^3).
+  const int cx = kTileX * (warps / 2), cy = kTileY * 2;
+  t.zr = kTileRun;
+  // the CTA's columns are at most `diag` voxels apart, and so are their
+  // in-plane coordinates rotated to any angle
+  const double diag = std::hypot((double)(cx - 1), (double)(cy - 1));
+  double fzmax = 0;
+  for (const Seg& s : p.seg) fzmax = std::max(fzmax, (double)std::fabs(s.fz));
+  // floor(x + d) - floor(x) <= floor(d) + 1; the 1e-3 covers float rounding
+  const double nb = std::floor(diag * p.fx_bp + 1e-3) + 3;
+  const double spread = std::floor(diag * fzmax + 1e-3) + 1;
+  const int ve = 16 / elem_bytes;
+  t.nb = (int)std::min((double)p.g.nrad, nb);
+  t.rows = (int)std::min((double)(p.g.nzs + 2), (double)t.zr + spread + 2);
+  // bins 4 words apart modulo 8 (16-byte copies, few bank conflicts)
+  int words = ((t.rows + 2 * (ve - 1)) * elem_bytes + 3) / 4;
+  words += (12 - words % 8) % 8;
+  t.rs = words * 4 / elem_bytes;
+  t.mw = (t.rows + 62) / 32 + 2;
+  t.rows_at = (48 + 4 * t.nb * t.mw + 15) / 16 * 16;
+  t.slot_bytes = (t.rows_at + (bp_pad_front(t.zr, elem_bytes) + t.nb * t.rs + t.zr + 2) * elem_bytes + 15) / 16 * 16;
+  return t;
+}
+
+// Tiles where their 8-warp CTAs (16 x 16 columns, one run) give about every SM
+// one; below, a view's latency shows and one warp per column is faster.
+// Columns / tiles, us a launch, by the number of CTAs: 54 / 95 at 48 CTAs (64 x
+// 64 x 32), 68 / 89 at 96 (64^3), 171 / 202 at 126 (48 x 48 x 159), 153 / 102
+// at 150 (72^3), 134 / 104 at 192 (128 x 128 x 32), 350 / 197 at 288 (96^3),
+// 1120 / 535 at 896 (128 x 128 x 159).
+bool bp_uses_tiles(const Plan& p) {
+  const BpTile t = tile_shape(p, 8, 4);  // the largest of its slots
+  if (2ll * t.warps * t.slot_bytes + 32ll * p.amax > 160 * 1024) return false;
+  const int b = (p.g.res + 15) / 16;
+  return b * b * ((p.g.nzs + kTileRun - 1) / kTileRun) >= 150;
+}
+
+BpTile bp_tile(const Plan& p, int warps, int elem_bytes) {
+  BpTile t = tile_shape(p, warps, elem_bytes);
+  if (!bp_uses_tiles(p)) t.zr = 0;
+  t.pads = bp_fast_pads(p);
+  return t;
+}
+
 int fp_default_R(const Plan& p) {
   for (int R : {9, 17, 25, 33}) {
     FpSchedule f;

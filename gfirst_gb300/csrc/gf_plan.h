@@ -79,6 +79,28 @@ struct BpPads {
 };
 BpPads bp_fast_pads(const Plan& p);
 
+// Shape of the back projector's work.  Column tiles (gf_bp_tile.cu): a warp owns
+// kTileX x kTileY columns and a run of zr = kTileRun slices, a CTA `warps` such
+// tiles (two in y) and one run.  zr = 0: one warp per column (gf_bp.cu), `warps`
+// a block.
+constexpr int kTileX = 4, kTileY = 8, kTileRun = 12;
+// Elements before a staged view's first row: a lane's run may start that far
+// before the segment's rows.
+constexpr int bp_pad_front(int zr, int elem_bytes) {
+  return (zr + 16 / elem_bytes - 1) / (16 / elem_bytes) * (16 / elem_bytes);
+}
+struct BpTile {
+  int zr = 0, warps = 0;
+  int nb = 0, rows = 0;     // radial bins and rows of one view at most
+  int rs = 0, mw = 0;       // row stride of a bin (elements), mask words of a bin
+  int rows_at = 0, slot_bytes = 0;
+  BpPads pads;              // one warp per column
+};
+// Whether a plan's back projections run as column tiles: a property of the
+// plan alone, since the sinogram layouts of a reconstruction follow from it.
+bool bp_uses_tiles(const Plan& p);
+BpTile bp_tile(const Plan& p, int warps, int elem_bytes);
+
 // Sinogram bin of (segment, plane, angle, radial), GFIRST.cu:175-176.
 inline int64_t lor_index(const Plan& p, int s, int iz0, int t, int r) {
   return ((int64_t)(iz0 - p.seg[s].zmin) + p.seg[s].acc) * ((int64_t)p.g.nrad * p.g.nang) + (int64_t)t * p.g.nrad + r;

@@ -5,7 +5,7 @@
 // in HBM for the whole reconstruction and a sub-iteration is a fixed chain
 // of kernels on one stream:
 //   psf    = XY PSF of the current image                      (GFIRST.cu:324-340)
-//   FP     = forward projection + ratio -> (corr, calib)       (GFIRST.cu:346-430)
+//   FP     = forward projection + ratio -> corr                (GFIRST.cu:346-430)
 //            [VLOR triples: FP -> split -> ratio, GFIRST.cu:373-430]
 //   BP     = back projection -> NUMER, DENOM                   (GFIRST.cu:436-469)
 //   update = ratio, XY PSF, axial filter, multiply, edges      (GFIRST.cu:482-502)
@@ -106,19 +106,18 @@ gf_status gf_recon::subiteration(int t, int s) {
     stage_begin(GF_STAGE_VLOR);
     GF_CK(cudaMemsetAsync(datos_v, 0, (size_t)pl.ndata * sizeof(float), st));
     GF_LAUNCH(c, launch_vlor_split_sorted(c->dg, vlor_keys, nev, events, proj_t, blankt, vlor_share, datos_v, st));
-    GF_LAUNCH(c, launch_ratio_gather(c->dg, c->d_rowmap, s, na, proj_t, datos_v, dbg[1] + off, cal + off, corrcal,
-                                     p.storage, st));
+    GF_LAUNCH(c, launch_ratio_gather(c->dg, c->d_rowmap, s, na, proj_t, datos_v, dbg[1] + off, cal_of(s), corr, p.storage, st));
     stage_end();
   } else {
     a.fr[0].dbg = dbg[t] + off;
-    a.fr[0].cal = cal + off;
-    a.fr[0].corrcal = corrcal;
+    a.fr[0].cal = cal_of(s);
+    a.fr[0].corr = corr;
     a.storage = p.storage;
     stage_begin(GF_STAGE_FP);
     GF_LAUNCH(c, launch_fp(a, c->fps, st));
     stage_end();
   }
-  BpArgs b = c->bp_args(s, corrcal, ratio, nullptr, p.storage);
+  BpArgs b = c->bp_args(s, bp_frame(s), p.storage);
   b.ratio = 1;
   // Triples data are mostly zero, and where a ratio of exactly 0 meets a
   // sentinel row the gap rule (GFIRST_GPU_Kernels.cu:157) turns on whether an
@@ -126,7 +125,7 @@ gf_status gf_recon::subiteration(int t, int s) {
   // reference's per-voxel rounding, or it drifts by ~1e-3 from it.
   if (t == 1) b.fast = 0;
   stage_begin(GF_STAGE_BP);
-  GF_LAUNCH(c, launch_bp(b, c->bp_warps, st));
+  GF_LAUNCH(c, launch_bp(b, c->bp_tile(p.storage), st));
   stage_end();
   stage_begin(GF_STAGE_UPDATE);
   GF_LAUNCH(c, launch_update(c->dg, ratio, g_bw, g5, img[t], st, store(t)));
@@ -170,7 +169,7 @@ bool fusable(const gf_recon* a, const gf_recon* b) {
          x->fps.R == y->fps.R && x->fps.lc == y->fps.lc;
 }
 
-gf_status fused_subiteration(gf_recon* const* G, int nfr, const int* cls, cudaStream_t st) {
+gf_status fused_subiteration(gf_recon* const* G, int nfr, cudaStream_t st) {
   if (nfr < 1 || nfr > kMaxFrames) return set_error(GF_ERR_ARG, "fused group size out of range");
   gf_recon* r0 = G[0];
   gf_ctx* c = r0->ctx;
@@ -192,48 +191,26 @@ gf_status fused_subiteration(gf_recon* const* G, int nfr, const int* cls, cudaSt
   for (int k = 0; k < nfr; k++) {
     const Plan& pk = G[k]->ctx->plan;
     const int64_t off = pk.sub_off[s];
-    a.fr[k] = FpFrame{G[k]->psf, G[k]->dbg[0] + off, G[k]->cal + off, G[k]->corrcal, nullptr, s, pk.nsub,
-                      pk.sub_nang[s]};
+    a.fr[k] = FpFrame{G[k]->psf, G[k]->dbg[0] + off, G[k]->cal_of(s), G[k]->corr, nullptr, s, pk.nsub, pk.sub_nang[s]};
   }
   GF_LAUNCH(c, launch_fp(a, c->fps, st));
   // the back projector keeps the subset a launch constant: one launch per
-  // subset count among the frames; within it, frames of one class (same
-  // normalization mask) share a warp per column two by two
+  // subset count among the frames
   std::vector<bool> done(nfr, false);
   for (int k0 = 0; k0 < nfr; k0++) {
     if (done[k0]) continue;
     const Plan& pl = G[k0]->ctx->plan;
-    BpArgs b = c->bp_args(s, nullptr, nullptr, nullptr, r0->p.storage);
+    BpArgs b = c->bp_args(s, BpFrame{}, r0->p.storage);
     b.g.nsub = pl.nsub;
     b.na = pl.sub_nang[s];
     b.ratio = 1;
-    std::vector<int> pairs, singles;
+    b.nfr = 0;
     for (int k = k0; k < nfr; k++) {
       if (done[k] || G[k]->ctx->plan.nsub != pl.nsub) continue;
       done[k] = true;
-      int j = -1;
-      if (b.fast && cls && cls[k] >= 0)
-        for (int m = k + 1; m < nfr && j < 0; m++)
-          if (!done[m] && cls[m] == cls[k]) j = m;
-      if (j >= 0) {
-        done[j] = true;
-        pairs.push_back(k);
-        pairs.push_back(j);
-      } else {
-        singles.push_back(k);
-      }
+      b.fr[b.nfr++] = G[k]->bp_frame(s);
     }
-    if (!pairs.empty()) {
-      b.nfr = (int)pairs.size();
-      for (size_t i = 0; i < pairs.size(); i++) b.fr[i] = BpFrame{G[pairs[i]]->corrcal, G[pairs[i]]->ratio, nullptr};
-      GF_LAUNCH(c, launch_bp_pairs(b, c->bp_warps, st));
-    }
-    if (!singles.empty()) {
-      b.nfr = (int)singles.size();
-      for (size_t i = 0; i < singles.size(); i++)
-        b.fr[i] = BpFrame{G[singles[i]]->corrcal, G[singles[i]]->ratio, nullptr};
-      GF_LAUNCH(c, launch_bp(b, c->bp_warps, st));
-    }
+    GF_LAUNCH(c, launch_bp(b, c->bp_tile(r0->p.storage), st));
   }
   ImgFrames u{};
   for (int k = 0; k < nfr; k++) u.fr[k] = ImgFrame{G[k]->ratio, nullptr, G[k]->img[0]};
@@ -296,10 +273,15 @@ gf_status gf_recon_create(gf_ctx* c, const gf_recon_params* prm, gf_recon** out)
       return fail(st);
     ALLOC(r->psf, pl.nvoxp);
     ALLOC(r->ratio, pl.nvoxp);
-    if ((st = r->alloc((size_t)pl.amax * pl.g.nrad * pl.PS * (prm->storage == GF_STORE_F32 ? 8 : 4), &r->corrcal)) != GF_OK)
-      return fail(st);
+    const size_t elem = (bp_uses_tiles(pl) ? 1 : 2) * (prm->storage == GF_STORE_F32 ? 4 : 2);
+    if ((st = r->alloc((size_t)pl.amax * pl.g.nrad * pl.PS * elem, &r->corr)) != GF_OK) return fail(st);
     ALLOC(r->dbg[0], pl.all_elems());
-    ALLOC(r->cal, pl.all_elems());
+    if (bp_uses_tiles(pl)) {
+      ALLOC(r->mask, r->mask_words());
+      ALLOC(r->dirty, r->dirty_words());
+    } else {
+      ALLOC(r->cal, pl.all_elems());
+    }
   }
   if (prm->mode >= 2) {
     ALLOC(r->dbg[1], pl.all_elems());
@@ -399,7 +381,12 @@ static gf_status load_impl(gf_recon* r, const float* h_image, const float* h_dsi
   if ((s = ck(cudaEventRecord(r->ev_staged, cs), "record staging")) != GF_OK) return done(s);
   if ((s = ck(cudaStreamWaitEvent(st, r->ev_staged, 0), "wait upload")) != GF_OK) return done(s);
   if ((s = ck(launch_build_dbg(c->dg, c->d_rowmap, s2, r->dbg[0], st), "build data")) != GF_OK) return done(s);
-  if ((s = ck(launch_build_cal(c->dg, c->d_rowmap, r->proj_ref, sn, r->cal, st), "build mask")) != GF_OK) return done(s);
+  if (r->cal) {
+    if ((s = ck(launch_build_cal(c->dg, c->d_rowmap, r->proj_ref, sn, r->cal, st), "build mask")) != GF_OK) return done(s);
+  } else {
+    if ((s = ck(cudaMemsetAsync(r->dirty, 0, r->dirty_words() * sizeof(unsigned), st), "memset")) != GF_OK) return done(s);
+    if ((s = ck(launch_build_mask(c->dg, c->d_rowmap, r->proj_ref, sn, r->mask, r->dirty, st), "build mask")) != GF_OK) return done(s);
+  }
   if (mode >= 2) {
     if ((s = ck(cudaMemcpyAsync(s2, h_tsino, 2 * pl.ndata * sizeof(float), cudaMemcpyHostToDevice, st), "upload triples")) != GF_OK) return done(s);
     if ((s = ck(launch_build_dbg(c->dg, c->d_rowmap, s2, r->dbg[1], st), "build triples")) != GF_OK) return done(s);

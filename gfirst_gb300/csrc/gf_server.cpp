@@ -270,8 +270,10 @@ gf_status gf_recon_bytes(const gf_geometry* gg, int32_t nsub, const gf_recon_par
     b += pl.nvox * 4;  // staging
   } else {
     b += 3 * v;                                                                   // second image, psf, ratio
-    b += (int64_t)pl.amax * pl.g.nrad * pl.PS * (p->storage == GF_STORE_F32 ? 8 : 4);  // ratio sinogram
-    b += all * 8 + all * 4;                                                       // data/background, mask
+    const bool tiles = bp_uses_tiles(pl);
+    b += (int64_t)pl.amax * pl.g.nrad * pl.PS * (tiles ? 1 : 2) * (p->storage == GF_STORE_F32 ? 4 : 2);  // ratio sinogram
+    b += all * 8;                                                                 // data/background
+    b += tiles ? all / 8 + (int64_t)pl.g.nang * pl.g.nrad * ((pl.g.nseg + 31) / 32) * 4 : all * 4;  // mask
     b += 3 * d;                                                                   // staging
   }
   if (p->mode >= 2) b += all * 8 + v;

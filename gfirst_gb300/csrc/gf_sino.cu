@@ -122,6 +122,61 @@ cudaError_t launch_build_cal(const DevGeom& g, const int2* rowmap, const float* 
   return cudaGetLastError();
 }
 
+// One word of mask bits per (angle row, radial bin, 32 padded rows), lane =
+// row, and the dirty bits: segments with a masked plane in this word.  at: the
+// (angle row, radial bin) index.
+__device__ __forceinline__ void put_mask_word(const DevGeom& g, const int2* __restrict__ rowmap, size_t at, int p0,
+                                              int lane, bool bit, unsigned* mask, unsigned* dirty) {
+  const unsigned word = __ballot_sync(0xffffffffu, bit);
+  if (lane == 0) mask[at * (g.PS >> 5) + (p0 >> 5)] = word;
+  const int2 m = p0 + lane < g.PS ? rowmap[p0 + lane] : make_int2(-1, -1);
+  const int nsw = (g.nseg + 31) >> 5;
+  const bool real = m.x >= 0 && m.y >= 0;
+  unsigned pend = __ballot_sync(0xffffffffu, real && !bit);
+  while (pend) {  // one atomic per segment in the word
+    const int seg = __shfl_sync(0xffffffffu, m.x, __ffs(pend) - 1);
+    if (lane == 0) atomicOr(dirty + at * nsw + (seg >> 5), 1u << (seg & 31));
+    pend &= ~__ballot_sync(0xffffffffu, real && m.x == seg);
+  }
+}
+
+// Normalization mask bits, GFIRST.cu:447, 453-458: 1 where proj_blank > 0.01
+// and blank > 0.01; oblique pad rows 0, segment 0's pad rows repeat its
+// first/last plane.
+__global__ void __launch_bounds__(256) build_mask_kernel(const DevGeom g, const int2* __restrict__ rowmap,
+                                                         const float* __restrict__ proj_ref,
+                                                         const float* __restrict__ norm, unsigned* mask,
+                                                         unsigned* dirty) {
+  __shared__ unsigned char tile[32][36];
+  const int r0 = blockIdx.x * 32, p0 = blockIdx.y * 32, theta = blockIdx.z;
+  const int tx = threadIdx.x, ty = threadIdx.y;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const int p = p0 + ty + 8 * k, r = r0 + tx;
+    bool v = false;
+    int seg, plane;
+    if (p < g.PS && r < g.nrad && resolve_row(g, rowmap[p], &seg, &plane)) {
+      const size_t lor = file_lor(g, seg, plane, theta, r);
+      v = (double)proj_ref[lor] > 0.01 && (double)norm[lor] > 0.01;
+    }
+    tile[ty + 8 * k][tx] = v;
+  }
+  __syncthreads();
+  const size_t base = (size_t)angle_rank(g, theta) * g.nrad;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const int r = r0 + ty + 8 * k;
+    if (r < g.nrad) put_mask_word(g, rowmap, base + r, p0, tx, tile[tx][ty + 8 * k] != 0, mask, dirty);
+  }
+}
+
+cudaError_t launch_build_mask(const DevGeom& g, const int2* rowmap, const float* proj_ref, const float* norm,
+                              unsigned* mask, unsigned* dirty, cudaStream_t st) {
+  const dim3 grid((g.nrad + 31) / 32, g.PS / 32, g.nang);
+  build_mask_kernel<<<grid, dim3(32, 8), 0, st>>>(g, rowmap, proj_ref, norm, mask, dirty);
+  return cudaGetLastError();
+}
+
 __device__ __forceinline__ float ratio_rule(float proj, float data, float bg) {
   // GFIRST.cu:423-429
   if ((double)bg < 0.) bg = 0.f;
@@ -129,39 +184,76 @@ __device__ __forceinline__ float ratio_rule(float proj, float data, float bg) {
   return (s >= 0.01f) ? __fdiv_rn(data, s) : -1000.f;
 }
 
-// (corr, calib) pairs of one subset from file-layout corr and calib.
-__global__ void corrcal_from_file_kernel(const DevGeom g, const int2* __restrict__ rowmap, int subset,
-                                         const float* __restrict__ corr, const float* __restrict__ calib,
-                                         float2* __restrict__ cc, size_t n) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int p = (int)(i % g.PS);
-  const size_t q = i / g.PS;
-  const int r = (int)(q % g.nrad), tl = (int)(q / g.nrad);
+// One subset from the file layout (gf_back_project), moved in 32x32 tiles as
+// above; pad rows of oblique segments hold the gap value.  PAIRS: (ratio, mask)
+// pairs, where *general is set (null: always); else ratios, mask bits, dirty
+// bits and *general = 1 where a mask value is neither 1 nor -1000.
+template <bool PAIRS>
+__global__ void __launch_bounds__(256) ratio_from_file_kernel(const DevGeom g, const int2* __restrict__ rowmap,
+                                                              int subset, const float* __restrict__ corr,
+                                                              const float* __restrict__ calib, void* out,
+                                                              unsigned* mask, unsigned* dirty, int* general) {
+  if (PAIRS && general && !*general) return;
+  __shared__ float tc[32][33], tm[32][33];
+  const int r0 = blockIdx.x * 32, p0 = blockIdx.y * 32, tl = blockIdx.z;
   const int theta = subset_angle(g, subset, tl);
-  int seg, plane;
-  float2 v = make_float2(-1000.f, -1000.f);
-  if (resolve_row(g, rowmap[p], &seg, &plane)) {
-    const size_t lor = file_lor(g, seg, plane, theta, r);
-    v = make_float2(corr[lor], calib[lor]);
+  const int tx = threadIdx.x, ty = threadIdx.y;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const int p = p0 + ty + 8 * k, r = r0 + tx;
+    float c = -1000.f, m = -1000.f;
+    int seg, plane;
+    if (p < g.PS && r < g.nrad && resolve_row(g, rowmap[p], &seg, &plane)) {
+      const size_t lor = file_lor(g, seg, plane, theta, r);
+      c = corr[lor];
+      m = calib[lor];
+    }
+    tc[ty + 8 * k][tx] = c;
+    tm[ty + 8 * k][tx] = m;
   }
-  cc[i] = v;
+  __syncthreads();
+  bool other = false;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const int r = r0 + ty + 8 * k;
+    if (r < g.nrad) {
+      const size_t at = (size_t)tl * g.nrad + r;
+      const float c = tc[tx][ty + 8 * k], m = tm[tx][ty + 8 * k];
+      if (PAIRS) {
+        static_cast<float2*>(out)[at * g.PS + p0 + tx] = make_float2(c, m);
+      } else {
+        static_cast<float*>(out)[at * g.PS + p0 + tx] = c;
+        other |= !(m == 1.f || m == -1000.f);
+        put_mask_word(g, rowmap, at, p0, tx, m == 1.f, mask, dirty);
+      }
+    }
+  }
+  if (!PAIRS && __any_sync(0xffffffffu, other) && tx == 0) *general = 1;
 }
 
-cudaError_t launch_corrcal_from_file(const DevGeom& g, const int2* rowmap, int subset, int na, const float* corr,
-                                     const float* calib, float2* corrcal, cudaStream_t st) {
-  const size_t n = (size_t)na * g.nrad * g.PS;
-  corrcal_from_file_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(g, rowmap, subset, corr, calib, corrcal, n);
+cudaError_t launch_ratio_from_file(const DevGeom& g, const int2* rowmap, int subset, int na, const float* corr,
+                                   const float* calib, float* out, unsigned* mask, unsigned* dirty, int* general,
+                                   cudaStream_t st) {
+  const dim3 grid((g.nrad + 31) / 32, g.PS / 32, na);
+  ratio_from_file_kernel<false><<<grid, dim3(32, 8), 0, st>>>(g, rowmap, subset, corr, calib, out, mask, dirty, general);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_pairs_from_file(const DevGeom& g, const int2* rowmap, int subset, int na, const float* corr,
+                                   const float* calib, float2* out, const int* general, cudaStream_t st) {
+  const dim3 grid((g.nrad + 31) / 32, g.PS / 32, na);
+  ratio_from_file_kernel<true><<<grid, dim3(32, 8), 0, st>>>(g, rowmap, subset, corr, calib, out, nullptr, nullptr,
+                                                             const_cast<int*>(general));
   return cudaGetLastError();
 }
 
 // Ratio for the VLOR triples (GFIRST.cu:415-430 with val_dato = datos_v*RES,
-// GFIRST.cu:397, 421) written as (corr, calib) pairs of one subset.
-template <class Pair>
+// GFIRST.cu:397, 421) of one subset, as ratios or, with cal, (ratio, mask) pairs.
+template <int STORE, bool PAIRS>
 __global__ void ratio_gather_kernel(const DevGeom g, const int2* __restrict__ rowmap, int subset,
                                     const float* __restrict__ proj_full, const float* __restrict__ datos_v,
                                     const float2* __restrict__ dbg_t, const float* __restrict__ cal,
-                                    Pair* __restrict__ cc, size_t n) {
+                                    void* __restrict__ out, size_t n) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int p = (int)(i % g.PS);
@@ -169,7 +261,7 @@ __global__ void ratio_gather_kernel(const DevGeom g, const int2* __restrict__ ro
   const int r = (int)(q % g.nrad), tl = (int)(q / g.nrad);
   const int theta = subset_angle(g, subset, tl);
   int seg, plane;
-  float2 v = make_float2(-1000.f, -1000.f);
+  float v = -1000.f, mask = -1000.f;
   const int2 m = rowmap[p];
   if (resolve_row(g, m, &seg, &plane)) {
     const size_t lor = file_lor(g, seg, plane, theta, r);
@@ -177,20 +269,28 @@ __global__ void ratio_gather_kernel(const DevGeom g, const int2* __restrict__ ro
     const int prow = (m.y >= 0) ? p : (m.y == -1 ? p + 1 : p - 1);
     const size_t e = i - p + prow;
     const float data = __fmul_rn(datos_v[lor], (float)g.res);
-    v = make_float2(ratio_rule(proj_full[lor], data, dbg_t[e].y), cal[e]);
+    v = ratio_rule(proj_full[lor], data, dbg_t[e].y);
+    if (PAIRS) mask = cal[e];
   }
-  cc[i] = pair_from<Pair>(v);
+  if constexpr (PAIRS) {
+    using P = typename PairT<STORE>::type;
+    static_cast<P*>(out)[i] = pair_from<P>(make_float2(v, mask));
+  } else {
+    using T = typename ElemT<STORE>::type;
+    static_cast<T*>(out)[i] = elem_from<T>(v);
+  }
 }
 
 cudaError_t launch_ratio_gather(const DevGeom& g, const int2* rowmap, int subset, int na, const float* proj_full,
-                                const float* datos_v, const float2* dbg_t, const float* cal, void* corrcal,
-                                int storage, cudaStream_t st) {
+                                const float* datos_v, const float2* dbg_t, const float* cal, void* out, int storage,
+                                cudaStream_t st) {
   const size_t n = (size_t)na * g.nrad * g.PS;
   const unsigned nb = (unsigned)((n + 255) / 256);
-  switch (storage) {
-    case 0: ratio_gather_kernel<<<nb, 256, 0, st>>>(g, rowmap, subset, proj_full, datos_v, dbg_t, cal, static_cast<float2*>(corrcal), n); break;
-    case 1: ratio_gather_kernel<<<nb, 256, 0, st>>>(g, rowmap, subset, proj_full, datos_v, dbg_t, cal, static_cast<__half2*>(corrcal), n); break;
-    case 2: ratio_gather_kernel<<<nb, 256, 0, st>>>(g, rowmap, subset, proj_full, datos_v, dbg_t, cal, static_cast<__nv_bfloat162*>(corrcal), n); break;
+  switch (storage * 2 + (cal ? 1 : 0)) {
+#define GF_RG(S, P) \
+  case S * 2 + P: ratio_gather_kernel<S, P><<<nb, 256, 0, st>>>(g, rowmap, subset, proj_full, datos_v, dbg_t, cal, out, n); break;
+    GF_RG(0, 0) GF_RG(0, 1) GF_RG(1, 0) GF_RG(1, 1) GF_RG(2, 0) GF_RG(2, 1)
+#undef GF_RG
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();

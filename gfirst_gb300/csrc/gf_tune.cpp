@@ -58,21 +58,21 @@ extern "C" gf_status gf_tune(gf_ctx* c, int32_t* fp_run, int32_t* fp_chunk, int3
   const Plan& p = c->plan;
   const size_t nsub0 = (size_t)p.sub_nang[0] * p.g.nrad * p.PS;
   float2* dbg = nullptr;
-  float* cal = nullptr;
+  float* cal = nullptr;  // mask of the (ratio, mask) pairs, where the back projector takes those
   GF_CK(cudaMallocAsync(&dbg, nsub0 * sizeof(float2), c->stream));
-  if (cudaMallocAsync(&cal, nsub0 * sizeof(float), c->stream) != cudaSuccess) {
-    cudaFreeAsync(dbg, c->stream);
-    return cuda_error(cudaGetLastError(), "cudaMallocAsync (tune)");
-  }
   auto done = [&](gf_status s) {
     cudaFreeAsync(dbg, c->stream);
-    cudaFreeAsync(cal, c->stream);
+    if (cal) cudaFreeAsync(cal, c->stream);
     cudaStreamSynchronize(c->stream);
     return s;
   };
   cudaStream_t st = c->stream;
   cudaError_t e = cudaMemsetAsync(dbg, 0, nsub0 * sizeof(float2), st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(cal, 0, nsub0 * sizeof(float), st);
+  const bool tiles = bp_uses_tiles(p);
+  if (e == cudaSuccess && tiles) e = cudaMemsetAsync(c->s_mask, 0xff, nsub0 / 8, st);
+  if (e == cudaSuccess && tiles) e = cudaMemsetAsync(c->s_dirty, 0, c->s_dirty_words() * sizeof(unsigned), st);
+  if (e == cudaSuccess && !tiles) e = cudaMallocAsync(&cal, nsub0 * sizeof(float), st);
+  if (e == cudaSuccess && !tiles) e = cudaMemsetAsync(cal, 0, nsub0 * sizeof(float), st);
   if (e == cudaSuccess) e = launch_cylinder(c->dg, 1.0f, c->s_img, st);
   if (e != cudaSuccess) return done(cuda_error(e, "tune set-up"));
   Timer tm;
@@ -104,7 +104,7 @@ extern "C" gf_status gf_tune(gf_ctx* c, int32_t* fp_run, int32_t* fp_chunk, int3
       a.lc = f.lc;
       a.fr[0].dbg = dbg;
       a.fr[0].cal = cal;
-      a.fr[0].corrcal = c->s_cc;
+      a.fr[0].corr = c->s_pairs;
       float ms = 0.f;
       s = time_it([&] { return launch_fp(a, f, st); }, &ms);
       if (s != GF_OK) return done(s);
@@ -122,9 +122,9 @@ extern "C" gf_status gf_tune(gf_ctx* c, int32_t* fp_run, int32_t* fp_chunk, int3
   int best_w = c->bp_warps;
   float best_bp = 3.0e38f;
   for (int w : {4, 8}) {
-    BpArgs b = c->bp_args(0, c->s_cc, c->s_numer, c->s_denom, 0);
+    BpArgs b = c->bp_args(0, BpFrame{c->s_pairs, c->s_mask, c->s_dirty, c->s_numer, c->s_denom}, 0);
     float ms = 0.f;
-    s = time_it([&] { return launch_bp(b, w, st); }, &ms);
+    s = time_it([&] { return launch_bp(b, bp_tile(p, w, 4), st); }, &ms);
     if (s != GF_OK) return done(s);
     c->launches += 4;
     if (ms < best_bp) {

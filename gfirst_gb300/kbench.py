@@ -5,8 +5,8 @@
 
 Runs a mode-1 reconstruction's stages on synthetic data and reports the
 device time per launch from the library's own stage events.  With --pairs,
-two frames of one normalization run as a fused group instead (the paired
-back projector), timed per frame and iteration on the host clock.  Small
+two frames of one normalization run as a fused group instead, timed per frame
+and iteration on the host clock.  Small
 enough to run under a profiler (one context, a few launches).
 """
 from __future__ import annotations

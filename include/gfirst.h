@@ -90,8 +90,7 @@ gf_status gf_synchronize(gf_ctx* ctx);
  * axial fraction of yrot*fz once per (column, view) for all voxels of the
  * column -- an interpolation weight moves by at most one unit in the last
  * place of iz + yrot*fz (about 1e-5 relative in the sums) -- and lets voxels
- * outside the segment's planes fall to the gap rule through sentinel rows
- * instead of a range test.  The reference's own hardware interpolation
+ * outside the segment's planes fall to the gap rule instead of a range test.  The reference's own hardware interpolation
  * quantises these weights to 1/256.  Default GF_BP_PER_VIEW.  The form
  * applies to gf_back_project and to the doubles image of reconstructions;
  * triples images (modes 2-3) always take GF_BP_PER_VOXEL: their data are
@@ -99,11 +98,11 @@ gf_status gf_synchronize(gf_ctx* ctx);
  * gap rule turns on whether a weight rounds to exactly 0. */
 enum { GF_BP_PER_VOXEL = 0, GF_BP_PER_VIEW = 1 };
 gf_status gf_set_bp_form(gf_ctx* ctx, int32_t form);
-/* The per-view form's staged-row buffer for a geometry (no device work): a
- * view's rows sit at offset pad_lo of rbuf (corr, calib) pairs per warp, the
- * rest hold the gap sentinel; pad_hi rows past a segment's last row are
- * read.  Shared memory per 4-warp block: 4 * (16 * angles per subset + 8 *
- * rbuf) bytes. */
+/* The per-view form's staged-row buffer for a geometry where it runs one warp
+ * per column (no device work): a view's rows sit at offset pad_lo of rbuf
+ * (corr, calib) pairs per warp, the rest hold the gap sentinel; pad_hi rows
+ * past a segment's last row are read.  Shared memory per 4-warp block: 4 *
+ * (16 * angles per subset + 8 * rbuf) bytes. */
 gf_status gf_bp_staged_rows(const gf_geometry* g, int32_t* pad_lo, int32_t* pad_hi, int32_t* rbuf);
 
 /* Device memory helpers for callers without a CUDA runtime of their own. */
@@ -285,16 +284,17 @@ gf_status gf_batch_synchronize(gf_batch* b);
  * frames that have a subset s, each at its own subset s; the forward PSF,
  * projection + ratio and update are one kernel launch over those frames and
  * the back projection one launch per subset count among them, each frame
- * keeping its own data and results (the same as alone, bit for bit).  With fused = 1, frames of a group with the
- * same subset count and equal normalization masks (checked on the device),
- * back projector in the per-view form, back-project two per warp, sharing
- * the per-view geometry and the staged mask rows; fused = 2 keeps one frame
- * per warp.  Other frames run on their own.  0 turns fusing off.  Takes
- * effect at the next iterate. */
+ * keeping its own data and results (the same as alone, bit for bit).  fused =
+ * 1 and 2 run the same launches; with 1, gf_batch_groups also compares the
+ * normalization masks of a group's frames (on the device) and counts the pairs
+ * of frames that share subset count and mask under the per-view form.  Other
+ * frames run on their own.  0 turns fusing off.  Takes effect at the next
+ * iterate. */
 gf_status gf_batch_set_fused(gf_batch* b, int32_t fused);
 /* Units the batch runs (fused groups and single frames), the size of the
- * largest group and the frame pairs back-projected together, as they stand
- * now (waits for the frames' queued work to compare their masks). */
+ * largest group and the pairs of frames of equal subset count and mask (fused
+ * = 1), as they stand now (waits for the frames' queued work to compare their
+ * masks). */
 gf_status gf_batch_groups(gf_batch* b, int32_t* units, int32_t* largest, int32_t* paired);
 
 /* ---- serving (no counterpart in the reference) ---------------------------- */
