@@ -4,37 +4,105 @@
 // (segment, angle) view with a blocking copy and a host scatter per launch
 // (GFIRST.cu:346-365), then the ratio loop of GFIRST.cu:413-430.
 //
-// GB300 design.  One CTA owns one (angle, radial bin) pair: every ray of that
-// pair, across all segments and planes, is parallel and shares the in-plane
-// sample positions (x, y) of each step lambda; only z differs.  So the CTA
-//  (1) resamples the image once per step onto a z column, B[lambda][z] =
-//      bilinear_xy(image[z], x(lambda), y(lambda)), reading the four z-fast
-//      image columns around (x, y) with coalesced loads (image in L2);
-//  (2) sums every ray of the pair from shared memory: ray (segment, plane
-//      iz0) at step lambda needs B[lambda] at z = iz0 + lambda*dz, a 1-D
-//      interpolation whose integer offset and fraction are the same for all
-//      planes of a segment, so a thread walks a run of R consecutive planes
-//      with R+1 shared loads and R interpolations per step;
-//  (3) applies the ratio in the epilogue and writes the ratios contiguously
-//      in the radial-major layout the back projector reads.
-// Work per ray-sample is one shared load and one 1-D interpolation instead of
+// GB300 design.  One CTA owns one angle and NB (1 or 4) neighbouring radial
+// bins: every ray of an (angle, bin) pair, across all segments and planes, is
+// parallel and shares the in-plane sample positions (x, y) of each step lambda;
+// only z differs.  So the CTA
+//  (1) resamples the image once per step onto a z column per bin, B[lambda][z]
+//      = bilinear_xy(image[z], x(lambda), y(lambda)), reading the four z-fast
+//      image columns around (x, y) with coalesced vector loads (image in L2);
+//  (2) sums every ray from shared memory: ray (segment, plane iz0) at step
+//      lambda needs B[lambda] at z = iz0 + lambda*dz, a 1-D interpolation whose
+//      integer offset and fraction are the same for all planes of a segment, so
+//      a thread walks a run of R consecutive planes with R+1 shared loads (of
+//      NB floats) and R interpolations per step, two bins at a time as packed
+//      FP32 operations;
+//  (3) passes the projections through shared memory into plane order, applies
+//      the ratio and writes the radial-major layout the back projector reads
+//      in whole lines.
+// Work per ray-sample is 1/NB shared loads and one 1-D interpolation instead of
 // eight texel reads; the image and data stream from HBM once.
+//
+// Bound: shared-memory wavefronts, a half of them conflicts between the
+// segments whose runs share a warp (NB = 1: 2.06 wavefronts per load; NB = 4,
+// where a load is served by quarter warps: 1.4).  128x128x159 voxels, 53
+// segments, 10 angles with the ratio 268 -> 250 us by resampling four slices a
+// thread and reading the data in whole lines; 15 segments, 21 angles 279 ->
+// 221; the whole sinogram of 168 angles x 1293 planes 1933 -> 1292 (four bins);
+// 64x64x32 voxels, 16 angles 36 -> 29.  Two bins a CTA (264, 222 with the
+// ratio) lost to either side of it.
+#include <algorithm>
+
 #include "gf_kernels.h"
 
 namespace gf {
 
+namespace {
+
+// The values of NB neighbouring radial bins at one sample or plane.
+template <int NB>
+struct alignas(4 * NB) Bins {
+  float v[NB];
+};
+
+// acc += a + w*(b - a), the sample's interpolation then the sum, each operation
+// rounded on its own; two bins at a time as packed operations (sm_100+ f32x2).
+template <int NB>
+__device__ __forceinline__ void add_sample(Bins<NB>& acc, const Bins<NB>& a, const Bins<NB>& b, float w) {
+  if constexpr (NB == 1) {
+    acc.v[0] += lerp_rn(a.v[0], b.v[0], w);
+  } else {
+#pragma unroll
+    for (int i = 0; i < NB; i += 2) {
+      const float2 a2 = make_float2(a.v[i], a.v[i + 1]);
+      float2 d;
+      asm("{\n\t.reg .b64 ra, rb, rc;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
+          "sub.rn.f32x2 rc, rb, ra;\n\tmov.b64 {%0, %1}, rc;\n\t}"
+          : "=f"(d.x), "=f"(d.y)
+          : "f"(a2.x), "f"(a2.y), "f"(b.v[i]), "f"(b.v[i + 1]));
+      const float2 s = __fadd2_rn(make_float2(acc.v[i], acc.v[i + 1]), __ffma2_rn(make_float2(w, w), d, a2));
+      acc.v[i] = s.x;
+      acc.v[i + 1] = s.y;
+    }
+  }
+}
+
+// NB consecutive floats from global memory (aligned to their size).
+template <int NB>
+__device__ __forceinline__ Bins<NB> ldg_bins(const float* p) {
+  Bins<NB> r;
+  if constexpr (NB == 1) {
+    r.v[0] = __ldg(p);
+  } else if constexpr (NB == 2) {
+    const float2 v = __ldg(reinterpret_cast<const float2*>(p));
+    r.v[0] = v.x;
+    r.v[1] = v.y;
+  } else {
+    const float4 v = __ldg(reinterpret_cast<const float4*>(p));
+    r.v[0] = v.x;
+    r.v[1] = v.y;
+    r.v[2] = v.z;
+    r.v[3] = v.w;
+  }
+  return r;
+}
+
+}  // namespace
+
 // PAIRS: the ratio output is (ratio, mask) pairs.
-template <int R, bool RATIO, bool FULL, int STORE, bool PAIRS>
-__global__ void __launch_bounds__(512) fp_kernel(const FpArgs a) {
+template <int R, int NB, bool RATIO, bool FULL, int STORE, bool PAIRS>
+__global__ void __launch_bounds__(512, R == 9 && NB == 1 ? 2 : 1) fp_kernel(const FpArgs a) {
+  using V = Bins<NB>;
+  constexpr int ZV = NB == 1 ? 4 : 2;  // slices resampled by a thread at a time
   extern __shared__ __align__(16) unsigned char smraw[];
   const int lc = a.lc, cw = a.cw;
-  int4* offs = reinterpret_cast<int4*>(smraw);              // [lc]
-  float2* wts = reinterpret_cast<float2*>(offs + lc);        // [lc]
-  float* col = reinterpret_cast<float*>(wts + lc);           // [lc][cw]
+  V* col = reinterpret_cast<V*>(smraw);                       // [lc][cw]
+  int4* offs = reinterpret_cast<int4*>(col + (size_t)lc * cw);  // [lc][NB]; cw is a multiple of 4
+  float2* wts = reinterpret_cast<float2*>(offs + lc * NB);    // [lc][NB]
 
   const DevGeom& g = a.g;
   const FpFrame& F = a.fr[blockIdx.z];
-  const int ird = blockIdx.x, tl = blockIdx.y;
+  const int ird = blockIdx.x * NB, tl = blockIdx.y;
   // a frame with fewer angles in its subset than the launch's largest: its
   // surplus blocks march no rays and write nothing (an early return here
   // costs the kernel 13 registers)
@@ -44,10 +112,6 @@ __global__ void __launch_bounds__(512) fp_kernel(const FpArgs a) {
   const int theta = subset_angle(F.subset, F.nsub, active ? tl : 0);
   const float2 sc = g.trig[theta];
   const float sn = sc.x, cs = sc.y;
-  // GFIRST_GPU_Kernels.cu:79-87 (fac = RES/NPT = 1 makes dx = sin, dy = -cos exactly)
-  const float x0 = __fmul_rn(g.fx_fp, __fsub_rn((float)ird, g.radm));
-  const float xc = __fadd_rn(__fadd_rn(g.resm, __fmul_rn(x0, cs)), 0.5f);
-  const float yc = __fadd_rn(__fadd_rn(g.resm, __fmul_rn(x0, sn)), 0.5f);
   const float dx = sn, dy = -cs;
   const int RES = g.res, NZS = g.nzs, NZP = g.nzp;
 
@@ -59,14 +123,22 @@ __global__ void __launch_bounds__(512) fp_kernel(const FpArgs a) {
     dz = g.seg[run.x].dz;
     zbase = a.padl + run.y;
   }
-  float acc[R];
+  V acc[R];
 #pragma unroll
-  for (int j = 0; j < R; j++) acc[j] = 0.f;
+  for (int j = 0; j < R; j++)
+#pragma unroll
+    for (int b = 0; b < NB; b++) acc[j].v[b] = 0.f;
 
   const int npad = cw - NZS;
   for (int lb = g.lam0; lb <= lam_end; lb += lc) {
     const int nl = min(lc, g.lam1 - lb + 1);
-    for (int l = tid; l < nl; l += nt) {
+    for (int e = tid; e < nl * NB; e += nt) {
+      const int l = e / NB, b = e - l * NB;
+      // GFIRST_GPU_Kernels.cu:79-87 (fac = RES/NPT = 1 makes dx = sin, dy = -cos exactly);
+      // a bin past the last one repeats it
+      const float x0 = __fmul_rn(g.fx_fp, __fsub_rn((float)min(ird + b, g.nrad - 1), g.radm));
+      const float xc = __fadd_rn(__fadd_rn(g.resm, __fmul_rn(x0, cs)), 0.5f);
+      const float yc = __fadd_rn(__fadd_rn(g.resm, __fmul_rn(x0, sn)), 0.5f);
       const float fl = (float)(lb + l);
       const float x = __fadd_rn(xc, __fmul_rn(fl, dx));
       const float y = __fadd_rn(yc, __fmul_rn(fl, dy));
@@ -75,27 +147,53 @@ __global__ void __launch_bounds__(512) fp_kernel(const FpArgs a) {
       const int i = (int)fx, j = (int)fy;
       const int i0 = clampi(i, 0, RES - 1), i1 = clampi(i + 1, 0, RES - 1);
       const int j0 = clampi(j, 0, RES - 1), j1 = clampi(j + 1, 0, RES - 1);
-      offs[l] = make_int4((j0 * RES + i0) * NZP, (j0 * RES + i1) * NZP, (j1 * RES + i0) * NZP, (j1 * RES + i1) * NZP);
-      wts[l] = make_float2(__fsub_rn(xb, fx), __fsub_rn(yb, fy));
+      offs[e] = make_int4((j0 * RES + i0) * NZP, (j0 * RES + i1) * NZP, (j1 * RES + i0) * NZP, (j1 * RES + i1) * NZP);
+      wts[e] = make_float2(__fsub_rn(xb, fx), __fsub_rn(yb, fy));
     }
     __syncthreads();
-    for (int idx = tid; idx < nl * NZP; idx += nt) {
-      const int l = idx / NZP, z = idx - l * NZP;
-      if (z < NZS) {
-        const int4 o = offs[l];
-        const float2 w = wts[l];
-        const float v00 = __ldg(F.img + o.x + z), v10 = __ldg(F.img + o.y + z);
-        const float v01 = __ldg(F.img + o.z + z), v11 = __ldg(F.img + o.w + z);
-        col[l * cw + a.padl + z] = lerp_rn(lerp_rn(v00, v10, w.x), lerp_rn(v01, v11, w.x), w.y);
+    // ZV slices a thread: one 4 ZV-byte load per corner column
+    const int nzq = NZP / ZV;
+    for (int idx = tid; idx < nl * nzq; idx += nt) {
+      const int l = (int)(((float)idx + 0.5f) * a.inv_nzq[ZV >> 1]), z = (idx - l * nzq) * ZV;
+      V c[ZV];
+#pragma unroll
+      for (int b = 0; b < NB; b++) {
+        const int4 o = offs[l * NB + b];
+        const float2 w = wts[l * NB + b];
+        const Bins<ZV> v00 = ldg_bins<ZV>(F.img + (o.x + z)), v10 = ldg_bins<ZV>(F.img + (o.y + z));
+        const Bins<ZV> v01 = ldg_bins<ZV>(F.img + (o.z + z)), v11 = ldg_bins<ZV>(F.img + (o.w + z));
+#pragma unroll
+        for (int k = 0; k < ZV; k++)
+          c[k].v[b] = lerp_rn(lerp_rn(v00.v[k], v10.v[k], w.x), lerp_rn(v01.v[k], v11.v[k], w.x), w.y);
+      }
+      V* to = col + l * cw + a.padl + z;
+      if (z + ZV <= NZS) {
+        if constexpr (NB * ZV <= 4) {
+          Bins<NB * ZV> q;
+#pragma unroll
+          for (int k = 0; k < ZV; k++)
+#pragma unroll
+            for (int b = 0; b < NB; b++) q.v[k * NB + b] = c[k].v[b];
+          *reinterpret_cast<Bins<NB * ZV>*>(to) = q;
+        } else {
+#pragma unroll
+          for (int k = 0; k < ZV; k++) to[k] = c[k];
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < ZV; k++)
+          if (z + k < NZS) to[k] = c[k];
       }
     }
     __syncthreads();
     if (npad > 0) {
-      for (int idx = tid; idx < nl * npad; idx += nt) {
-        const int l = idx / npad, p = idx - l * npad;
-        float* c = col + l * cw;
-        if (p < a.padl) c[p] = c[a.padl];
-        else c[a.padl + NZS + (p - a.padl)] = c[a.padl + NZS - 1];
+      for (int l = tid >> 5; l < nl; l += nt >> 5) {
+        V* c = col + l * cw;
+        const V lo = c[a.padl], hi = c[a.padl + NZS - 1];
+        for (int p = tid & 31; p < npad; p += 32) {
+          if (p < a.padl) c[p] = lo;
+          else c[NZS + p] = hi;
+        }
       }
       __syncthreads();
     }
@@ -104,12 +202,12 @@ __global__ void __launch_bounds__(512) fp_kernel(const FpArgs a) {
         const float t = __fmul_rn((float)(lb + l), dz);
         const float mf = floorf(t);
         const float f = __fsub_rn(t, mf);
-        const float* c = col + l * cw + zbase + (int)mf;
-        float va = c[0];
+        const V* c = col + l * cw + zbase + (int)mf;
+        V va = c[0];
 #pragma unroll
         for (int j = 0; j < R; j++) {
-          const float vb = c[j + 1];
-          acc[j] += lerp_rn(va, vb, f);
+          const V vb = c[j + 1];
+          add_sample(acc[j], va, vb, f);
           va = vb;
         }
       }
@@ -117,52 +215,102 @@ __global__ void __launch_bounds__(512) fp_kernel(const FpArgs a) {
     __syncthreads();
   }
 
-  if (run.x < 0 || !active) return;
-  const DevSeg sg = g.seg[run.x];
-  const size_t base = ((size_t)tl * g.nrad + ird) * g.PS;
+  if (!active) return;  // whole block
+  DevSeg sg{};
+  if (run.x >= 0) sg = g.seg[run.x];
+  const int plane = sg.acc + (run.y - sg.zmin);  // of the run's first ray
+  if constexpr (FULL) {
+    if (run.x < 0) return;
+    const size_t step = (size_t)g.nrad * g.nang;
+    float* to = F.proj_full + (size_t)plane * step + (size_t)theta * g.nrad + ird;
 #pragma unroll
-  for (int j = 0; j < R; j++) {
-    if (j < run.z) {
-      const int iz0 = run.y + j;
-      const float proj = acc[j];
-      if (FULL) {
-        const size_t lor = ((size_t)(iz0 - sg.zmin) + sg.acc) * ((size_t)g.nrad * g.nang) + (size_t)theta * g.nrad + ird;
-        F.proj_full[lor] = proj;
+    for (int j = 0; j < R; j++) {
+      if (j < run.z) {
+#pragma unroll
+        for (int b = 0; b < NB; b++)
+          if (NB == 1 || ird + b < g.nrad) to[(size_t)j * step + b] = acc[j].v[b];
       }
-      if (RATIO) {
-        const size_t o = base + sg.blk + 1 + (iz0 - sg.zmin);
-        const float2 db = F.dbg[o];
-        const float s = __fadd_rn(proj, db.y);
-        const float corr = (s >= 0.01f) ? __fdiv_rn(db.x, s) : -1000.f;
-        auto put = [&](auto* out, auto v, auto sentinel) {
-          out[o] = v;
-          if (j == 0 && (run.w & 1)) out[o - 1] = (run.x == 0) ? v : sentinel;
-          if (j == run.z - 1 && (run.w & 2)) out[o + 1] = (run.x == 0) ? v : sentinel;
-        };
+    }
+  }
+  if constexpr (RATIO) {
+    // the projections in plane order through shared memory, so that the data
+    // are read and the ratios written in whole lines
+    V* buf = reinterpret_cast<V*>(smraw);
+    if (run.x >= 0) {
+#pragma unroll
+      for (int j = 0; j < R; j++)
+        if (j < run.z) buf[plane + j] = acc[j];
+    }
+    __syncthreads();
+    const size_t base = ((size_t)tl * g.nrad + ird) * g.PS;
+    for (int p = tid; p < g.PP; p += nt) {
+      // pad rows: segment 0's repeat its first and last plane, the others are gaps
+      const int pl = a.rowplane[p];
+      const int row = p == 0 ? 1 : (p == NZS + 1 ? NZS : p);
+      V proj{};
+      if (pl >= 0) proj = buf[pl];
+#pragma unroll
+      for (int b = 0; b < NB; b++) {
+        if (NB > 1 && ird + b >= g.nrad) break;  // whole block
+        const size_t o = base + (size_t)b * g.PS;
+        float corr = -1000.f, cal = -1000.f;
+        if (pl >= 0) {
+          const float2 db = F.dbg[o + row];
+          const float s = __fadd_rn(proj.v[b], db.y);
+          corr = (s >= 0.01f) ? __fdiv_rn(db.x, s) : -1000.f;
+          if (PAIRS) cal = F.cal[o + row];
+        }
         if constexpr (PAIRS) {
           using P = typename PairT<STORE>::type;
-          put(static_cast<P*>(F.corr), pair_from<P>(make_float2(corr, F.cal[o])),
-              pair_from<P>(make_float2(-1000.f, -1000.f)));
+          static_cast<P*>(F.corr)[o + p] = pair_from<P>(make_float2(corr, cal));
         } else {
           using T = typename ElemT<STORE>::type;
-          put(static_cast<T*>(F.corr), elem_from<T>(corr), elem_from<T>(-1000.f));
+          static_cast<T*>(F.corr)[o + p] = elem_from<T>(corr);
         }
       }
     }
   }
 }
 
-template <int R, bool RATIO, bool FULL, int STORE, bool PAIRS>
-static cudaError_t launch_fp_t(const FpArgs& a, const FpSchedule& s, cudaStream_t st) {
-  auto k = fp_kernel<R, RATIO, FULL, STORE, PAIRS>;
-  size_t smem = s.smem_bytes();
+template <int R, int NB, bool RATIO, bool FULL, int STORE, bool PAIRS>
+static cudaError_t launch_fp_n(FpArgs a, const FpSchedule& s, int na, cudaStream_t st) {
+  auto k = fp_kernel<R, NB, RATIO, FULL, STORE, PAIRS>;
+  if (NB > 1) a.lc = (s.lc + 1) / 2;  // 64 KB of columns at the default 32 steps, as many bytes as 64 steps of one bin
+  size_t smem = (size_t)a.lc * a.cw * sizeof(Bins<NB>) + (size_t)a.lc * NB * (sizeof(int4) + sizeof(float2));
+  if (RATIO) smem = std::max(smem, (size_t)a.g.P * sizeof(Bins<NB>));
+  a.inv_nzq[0] = 1.f / (float)a.g.nzp;
+  a.inv_nzq[1] = 2.f / (float)a.g.nzp;
+  a.inv_nzq[2] = 4.f / (float)a.g.nzp;
   cudaError_t e = allow_max_smem(k);
   if (e != cudaSuccess) return e;
-  int na = 0;
-  for (int f = 0; f < (a.nfr > 1 ? a.nfr : 1); f++) na = a.fr[f].na > na ? a.fr[f].na : na;
-  dim3 grid(a.g.nrad, na, a.nfr > 1 ? a.nfr : 1);
+  dim3 grid((a.g.nrad + NB - 1) / NB, na, a.nfr > 1 ? a.nfr : 1);
   k<<<grid, s.nthreads, smem, st>>>(a);
   return cudaGetLastError();
+}
+
+// Bins per CTA.  Four bins share the loads' addresses, a quarter of the warp's
+// conflicts and packed arithmetic, but make a quarter of the CTAs with twice
+// the registers: they pay where the grid is large.  One / four bins, us a
+// launch, by the threads of the one-bin grid: projections (layout kernel
+// included) 27 / 37 at 33 K (64x64x32, 16 angles), 81 / 73 at 221 K (96^3, 12
+// angles), 273 / 273 at 655 K (128x128x159, 53 segments, 10 angles: 320 CTAs
+// on 152 SMs; 247 / 191 where the next call's CTAs fill the last wave), 228 /
+// 201 at 0.5 M and 1641 / 1292 at 4 M (15 segments, 21 and 168 angles).  With the
+// ratio, whose data the fewer warps wait for, 76 / 82, 252 / 292, 220 / 223 and
+// 1576 / 1419; eight frames of 96^3 in one launch lose 6 % to it, so a group of
+// frames stays at one bin.
+template <int R, bool RATIO, bool FULL, int STORE, bool PAIRS>
+static cudaError_t launch_fp_t(const FpArgs& a, const FpSchedule& s, cudaStream_t st) {
+  int na = 0;
+  for (int f = 0; f < (a.nfr > 1 ? a.nfr : 1); f++) na = a.fr[f].na > na ? a.fr[f].na : na;
+  if constexpr (R == 9) {
+    const long long threads = (long long)a.g.nrad * na * (a.nfr > 1 ? a.nfr : 1) * s.nthreads;
+    const size_t smem4 = (size_t)std::max((s.lc + 1) / 2 * (a.cw + 6), a.g.P) * sizeof(Bins<4>);
+    if (RATIO ? a.nfr <= 1 && threads >= 2000000 : threads >= 150000)
+      if (smem4 <= 200 * 1024)
+        return launch_fp_n<R, 4, RATIO, FULL, STORE, PAIRS>(a, s, na, st);
+  }
+  return launch_fp_n<R, 1, RATIO, FULL, STORE, PAIRS>(a, s, na, st);
 }
 
 template <int R, bool PAIRS>

@@ -60,6 +60,7 @@ struct gf_ctx {
   gf::DevSeg* d_seg = nullptr;
   float2* d_trig = nullptr;
   int2* d_rowmap = nullptr;
+  int* d_rowplane = nullptr;  // per padded row: FpArgs::rowplane
   int4* d_runs = nullptr;
   float* d_gtab = nullptr;
   float gtab_sigma = -1.f;

@@ -108,10 +108,11 @@ bool make_fp_schedule(const Plan& p, int R, int lc, FpSchedule* out) {
   }
   f.nthreads = ((int)f.runs.size() + 31) / 32 * 32;
   if (f.nthreads > 512) return false;
-  f.padl = -kmin;
+  f.padl = (-kmin + 3) / 4 * 4;  // slice 0 of a column on a 16-byte boundary
   f.padr = kmax - (p.g.nzs - 1);
-  f.cw = f.padl + p.g.nzs + f.padr;
+  f.cw = p.g.nzs + f.padr - kmin;
   if (f.smem_bytes() > 200 * 1024) return false;
+  f.cw = (f.padl + p.g.nzs + f.padr + 3) / 4 * 4;  // at most 6 floats a step more, 6 KB at 256 steps
   *out = std::move(f);
   return true;
 }
