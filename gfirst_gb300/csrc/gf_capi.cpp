@@ -45,19 +45,6 @@ Taps5 gauss5() {
   return t;
 }
 
-std::vector<float> bilateral_table(float sigma3d) {
-  // float G = exp(-dist_spatial2/((2.0*sigma3D)*(2.0*sigma3D))), GFIRST_GPU_Kernels.cu:526-528
-  std::vector<float> t(729);
-  const double cs = (2.0 * (double)sigma3d) * (2.0 * (double)sigma3d);
-  for (int dz = -4; dz <= 4; dz++)
-    for (int dy = -4; dy <= 4; dy++)
-      for (int dx = -4; dx <= 4; dx++) {
-        float d2 = (float)(dx * dx + dy * dy + dz * dz);
-        t[((dz + 4) * 9 + (dy + 4)) * 9 + (dx + 4)] = (float)exp((double)(-d2) / cs);
-      }
-  return t;
-}
-
 static bool to_geom(const gf_geometry* g, Geom* out) {
   if (!g) return false;
   *out = Geom{g->res, g->nzs, g->nrad, g->nang, g->span, g->nseg, g->pitch_mm, g->diam_det_mm, g->fov_mm};
@@ -94,17 +81,6 @@ gf_status gf_ctx::ensure_scratch() {
   if (bp_uses_tiles(p)) {
     GF_TRY(alloc_t(n / 32, &s_mask));
     GF_TRY(alloc_t(s_dirty_words() + 1, &s_dirty));
-  }
-  return GF_OK;
-}
-
-gf_status gf_ctx::ensure_gtab(float sigma3d) {
-  if (!d_gtab) GF_TRY(alloc_t(729, &d_gtab));
-  if (gtab_sigma != sigma3d) {
-    std::vector<float> t = bilateral_table(sigma3d);
-    GF_CK(cudaMemcpyAsync(d_gtab, t.data(), 729 * sizeof(float), cudaMemcpyHostToDevice, stream));
-    GF_CK(cudaStreamSynchronize(stream));
-    gtab_sigma = sigma3d;
   }
   return GF_OK;
 }
@@ -549,10 +525,9 @@ gf_status gf_bilateral(gf_ctx* c, const float* d_in, const float* d_ref, float m
   if (!c || !d_in || !d_ref || !d_out) return set_error(GF_ERR_ARG, "null argument");
   if (r < 0 || r > 4) return set_error(GF_ERR_ARG, "window radius must be in [0, 4]");
   GF_TRY(c->ensure_scratch());
-  GF_TRY(c->ensure_gtab(sigma3d));
   GF_LAUNCH(c, launch_file_to_zfast(c->dg, d_in, c->s_img, c->stream));
   GF_LAUNCH(c, launch_file_to_zfast(c->dg, d_ref, c->s_img2, c->stream));
-  GF_LAUNCH(c, launch_bilateral(c->dg, c->s_img, c->s_img2, nullptr, max_ref, r, sigmai, c->d_gtab, c->s_numer, c->stream));
+  GF_LAUNCH(c, launch_bilateral(c->dg, c->s_img, c->s_img2, nullptr, max_ref, r, sigma3d, sigmai, c->s_numer, c->stream));
   GF_LAUNCH(c, launch_zfast_to_file(c->dg, c->s_numer, 1.f, 0, d_out, c->stream));
   return GF_OK;
 }

@@ -7,6 +7,8 @@
 // 508-539) and layout conversions.  All of these are HBM-bound except the
 // bilateral filter; they keep the reference's operation order with explicit
 // round-to-nearest arithmetic so their results equal the reference's.
+#include <cmath>
+
 #include "gf_kernels.h"
 
 namespace gf {
@@ -357,91 +359,152 @@ cudaError_t launch_max_nonneg(const DevGeom& g, const void* img, float* d_max, c
   return cudaGetLastError();
 }
 
+// 2^x, the special function unit's (0 below 2^-126)
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 // ---- joint bilateral filter, GFIRST_GPU_Kernels.cu:508-539 ---------------
-// CTA: 4x4 columns x 32 slices, reference and input staged with a halo of 4.
-// Voxels with a coordinate below r give 0 (the reference's unsigned window
-// start wraps and its loops run zero times).  Spatial weights come from a
-// table computed on the host exactly as the reference computes them
-// (double exp, stored as float); the intensity weight uses __expf in FP32
-// (the reference evaluates it in double) and the intensity difference is
-// scaled by 1/max_ref.
-constexpr int BL_T = 4, BL_H = 4;
-template <class T>
-__global__ void __launch_bounds__(512) bilateral_kernel(const DevGeom g, const T* __restrict__ in,
-                                                        const T* __restrict__ ref,
-                                                        const float* __restrict__ d_max_ref, float max_ref_host,
-                                                        int r, float neg_inv_ci, const float* __restrict__ gtab,
-                                                        float* __restrict__ out) {
-  constexpr int W = BL_T + 2 * BL_H;  // 12 columns
-  constexpr int ZW = 32 + 2 * BL_H;   // 40 slices
-  __shared__ float Sr[W][W][ZW + 1];
-  __shared__ float Si[W][W][ZW + 1];
+// CTA: 8x8 columns x 32 slices, reference and input staged with a halo of 4;
+// a thread owns one slice (its lane) of BL_N columns along x, so the BL_N + 2 R
+// values of a window row are loaded once for all of them.  Voxels with a
+// coordinate below R give 0 (the reference's unsigned window start wraps and
+// its loops run zero times); past the far sides the staged reference is
+// infinite, which makes the weight 0.  A tap's weight is exp of the intensity
+// and the x distance together, one ex2 of a fused multiply-add; the y and z
+// part of the spatial weight scales a row's two sums.  FP32 throughout, where
+// the reference evaluates its exponentials in double: 3e-7 from 64 bits on
+// 128x128x159 voxels (9e-7 with a weight of two factors).
+//
+// Bound: the 729 exponentials a voxel (16 a clock and SM: 377 us for 128x128x159
+// voxels), with instruction issue 86 % busy beside them.  gf_bilateral on
+// 128x128x159 voxels takes 449 us with its three layout kernels; one column a
+// thread, with a table lookup, five multiplications and two shared loads a tap,
+// took 1644.
+constexpr int BL_T = 8, BL_H = 4, BL_N = 4;
+constexpr int BL_W = BL_T + 2 * BL_H, BL_Z = 32 + 2 * BL_H + 1;  // staged columns a side, slices and one of padding
+constexpr size_t kBlSmem = (size_t)2 * BL_W * BL_W * BL_Z * sizeof(float);
+
+struct BlTaps {
+  float lx[BL_H + 1];  // log2 of the spatial weight at distance 0..BL_H along an axis
+};
+
+template <class T, int R>
+__global__ void __launch_bounds__(512, 2) bilateral_kernel(const DevGeom g, const T* __restrict__ in,
+                                                           const T* __restrict__ ref,
+                                                           const float* __restrict__ d_max_ref, float max_ref_host,
+                                                           float root_log2e_ci, const BlTaps taps,
+                                                           float* __restrict__ out) {
+  extern __shared__ float bl_smem[];
+  float* Sr = bl_smem;
+  float* Si = bl_smem + BL_W * BL_W * BL_Z;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int x0 = blockIdx.x * BL_T, y0 = blockIdx.y * BL_T, z0 = blockIdx.z * 32;
   const int RES = g.res, NZS = g.nzs, NZP = g.nzp;
-  for (int idx = threadIdx.x; idx < W * W * ZW; idx += blockDim.x) {
-    const int zz = idx % ZW, c = idx / ZW;
-    const int yy = c / W, xx = c % W;
-    const int y = y0 - BL_H + yy, x = x0 - BL_H + xx, z = z0 - BL_H + zz;
-    float vr = 0.f, vi = 0.f;
-    if (y >= 0 && y < RES && x >= 0 && x < RES && z >= 0 && z < NZS) {
-      const size_t o = ((size_t)y * RES + x) * NZP + z;
-      vr = img_ld(ref + o);
-      vi = img_ld(in + o);
+  for (int c = wid; c < BL_W * BL_W; c += 16) {
+    const int yy = c / BL_W, xx = c - yy * BL_W;
+    const int y = y0 - BL_H + yy, x = x0 - BL_H + xx;
+    const bool col = y >= 0 && y < RES && x >= 0 && x < RES;
+    const long long o = ((long long)y * RES + x) * NZP;
+    for (int zz = lane; zz < 32 + 2 * BL_H; zz += 32) {
+      const int z = z0 - BL_H + zz;
+      const bool ok = col && z >= 0 && z < NZS;
+      Sr[c * BL_Z + zz] = ok ? img_ld(ref + (o + z)) : __int_as_float(0x7f800000);
+      Si[c * BL_Z + zz] = ok ? img_ld(in + (o + z)) : 0.f;
     }
-    Sr[yy][xx][zz] = vr;
-    Si[yy][xx][zz] = vi;
   }
   __syncthreads();
-  const int ty = wid >> 2, tx = wid & 3;
-  const int y = y0 + ty, x = x0 + tx, z = z0 + lane;
-  if (y >= RES || x >= RES) return;
+  const int ty = wid >> 1, tx = (wid & 1) * BL_N;  // row, first column of the thread's
+  const int y = y0 + ty, z = z0 + lane;
+  if (y >= RES || x0 + tx >= RES) return;  // whole warp
   const float max_ref = d_max_ref ? *d_max_ref : max_ref_host;
-  const float rinv = 1.0f / max_ref;
-  float res = 0.f;
-  if (z < NZS && x >= r && y >= r && z >= r) {
-    const float ref0 = Sr[ty + BL_H][tx + BL_H][lane + BL_H];
-    float norm = 0.f, sum = 0.f;
-    for (int dz = -r; dz <= r; dz++) {
-      if (z + dz >= NZS) break;
-      for (int dy = -r; dy <= r; dy++) {
-        if (y + dy >= RES) break;
-        const float* rr = &Sr[ty + BL_H + dy][tx + BL_H][lane + BL_H + dz];
-        const float* ii = &Si[ty + BL_H + dy][tx + BL_H][lane + BL_H + dz];
-        const float* gw = gtab + ((dz + 4) * 9 + (dy + 4)) * 9 + 4;
-        for (int dx = -r; dx <= r; dx++) {
-          if (x + dx >= RES) break;
-          const float d = __fmul_rn(__fsub_rn(rr[dx * (ZW + 1)], ref0), rinv);
-          const float h = __expf(__fmul_rn(__fmul_rn(d, d), neg_inv_ci));
-          const float w = __fmul_rn(h, __ldg(gw + dx));
-          norm = __fadd_rn(norm, w);
-          sum = __fadd_rn(sum, __fmul_rn(w, ii[dx * (ZW + 1)]));
+  const float k = (1.0f / max_ref) * root_log2e_ci;  // exp(-(d / max_ref)^2 / ci) = 2^-(d k)^2
+  const int at = ((ty + BL_H) * BL_W + tx + BL_H) * BL_Z + lane + BL_H;
+  float ref0[BL_N], norm[BL_N], sum[BL_N];
+#pragma unroll
+  for (int n = 0; n < BL_N; n++) {
+    ref0[n] = Sr[at + n * BL_Z];
+    norm[n] = sum[n] = 0.f;
+  }
+#pragma unroll 1
+  for (int dz = -R; dz <= R; dz++) {
+#pragma unroll 1
+    for (int dy = -R; dy <= R; dy++) {
+      const int row = at + dy * BL_W * BL_Z + dz;
+      float r[BL_N + 2 * R], v[BL_N + 2 * R];
+#pragma unroll
+      for (int i = 0; i < BL_N + 2 * R; i++) {
+        r[i] = Sr[row + (i - R) * BL_Z];
+        v[i] = Si[row + (i - R) * BL_Z];
+      }
+      const float gyz = ex2(taps.lx[1] * (float)(dz * dz + dy * dy));
+#pragma unroll
+      for (int n = 0; n < BL_N; n++) {
+        float rn = 0.f, rs = 0.f;
+#pragma unroll
+        for (int i = 0; i <= 2 * R; i++) {
+          const float d = (r[n + i] - ref0[n]) * k;
+          const float w = ex2(__fmaf_rn(-d, d, taps.lx[i < R ? R - i : i - R]));
+          rn += w;
+          rs = __fmaf_rn(w, v[n + i], rs);
         }
+        norm[n] = __fmaf_rn(gyz, rn, norm[n]);
+        sum[n] = __fmaf_rn(gyz, rs, sum[n]);
       }
     }
-    res = ((double)norm > 1e-8) ? __fdiv_rn(sum, norm) : 0.f;
   }
-  out[((size_t)y * RES + x) * NZP + z] = (z < NZS) ? res : 0.f;
+#pragma unroll
+  for (int n = 0; n < BL_N; n++) {
+    const int x = x0 + tx + n;
+    if (x >= RES) break;  // whole warp
+    float res = 0.f;
+    if (z < NZS && x >= R && y >= R && z >= R) res = ((double)norm[n] > 1e-8) ? __fdiv_rn(sum[n], norm[n]) : 0.f;
+    out[((size_t)y * RES + x) * NZP + z] = res;
+  }
+}
+
+template <class T, int R>
+static cudaError_t launch_bilateral_r(const DevGeom& g, const void* in, const void* ref, const float* d_max_ref,
+                                      float max_ref, float root, const BlTaps& taps, float* out, cudaStream_t st) {
+  auto k = bilateral_kernel<T, R>;
+  cudaError_t e = allow_max_smem(k);
+  if (e != cudaSuccess) return e;
+  const dim3 grid((g.res + BL_T - 1) / BL_T, (g.res + BL_T - 1) / BL_T, g.nzp / 32);
+  k<<<grid, 512, kBlSmem, st>>>(g, static_cast<const T*>(in), static_cast<const T*>(ref), d_max_ref, max_ref, root, taps,
+                                out);
+  return cudaGetLastError();
+}
+
+template <class T>
+static cudaError_t launch_bilateral_t(int r, const DevGeom& g, const void* in, const void* ref, const float* d_max_ref,
+                                      float max_ref, float root, const BlTaps& taps, float* out, cudaStream_t st) {
+  switch (r) {
+    case 0: return launch_bilateral_r<T, 0>(g, in, ref, d_max_ref, max_ref, root, taps, out, st);
+    case 1: return launch_bilateral_r<T, 1>(g, in, ref, d_max_ref, max_ref, root, taps, out, st);
+    case 2: return launch_bilateral_r<T, 2>(g, in, ref, d_max_ref, max_ref, root, taps, out, st);
+    case 3: return launch_bilateral_r<T, 3>(g, in, ref, d_max_ref, max_ref, root, taps, out, st);
+    case 4: return launch_bilateral_r<T, 4>(g, in, ref, d_max_ref, max_ref, root, taps, out, st);
+    default: return cudaErrorInvalidValue;
+  }
 }
 
 cudaError_t launch_bilateral(const DevGeom& g, const void* in, const void* ref, const float* d_max_ref,
-                             float max_ref, int r, float sigmai, const float* gtab, float* out, cudaStream_t st,
+                             float max_ref, int r, float sigma3d, float sigmai, float* out, cudaStream_t st,
                              int store) {
-  if (r < 0 || r > BL_H) return cudaErrorInvalidValue;
   const double ci = (2.0 * (double)sigmai) * (2.0 * (double)sigmai);
-  const float neg_inv_ci = (float)(-1.0 / ci);
-  dim3 grid((g.res + BL_T - 1) / BL_T, (g.res + BL_T - 1) / BL_T, g.nzp / 32);
+  const double cs = (2.0 * (double)sigma3d) * (2.0 * (double)sigma3d);
+  const double log2e = 1.4426950408889634;
+  BlTaps t;
+  for (int i = 0; i <= BL_H; i++) t.lx[i] = (float)fmax(-1e30, -(double)(i * i) / cs * log2e);
+  const float root = (float)sqrt(log2e / ci);
   switch (store) {
-#define GF_BL(S, T)                                                                                        \
-  case S:                                                                                                  \
-    bilateral_kernel<<<grid, 512, 0, st>>>(g, static_cast<const T*>(in), static_cast<const T*>(ref),     \
-                                           d_max_ref, max_ref, r, neg_inv_ci, gtab, out);                 \
-    break;
-    GF_BL(0, float) GF_BL(1, __half) GF_BL(2, __nv_bfloat16)
-#undef GF_BL
+    case 0: return launch_bilateral_t<float>(r, g, in, ref, d_max_ref, max_ref, root, t, out, st);
+    case 1: return launch_bilateral_t<__half>(r, g, in, ref, d_max_ref, max_ref, root, t, out, st);
+    case 2: return launch_bilateral_t<__nv_bfloat16>(r, g, in, ref, d_max_ref, max_ref, root, t, out, st);
     default: return cudaErrorInvalidValue;
   }
-  return cudaGetLastError();
 }
 
 // img2 = (1.0 - 0.1f)*img2 + 0.1f*filtered, GFIRST.cu:524 (double, as there).

@@ -36,7 +36,6 @@ gf_status cuda_error(cudaError_t e, const char* what);
 
 Taps9 gauss9(float psf);   // calcGaussianCoefficients, GFIRST_GPU_Kernels.cu:322-330
 Taps5 gauss5();            // gaussian_filterZ's taps, GFIRST_CPU_Kernels.cpp:169-173
-std::vector<float> bilateral_table(float sigma3d);  // 9x9x9 spatial weights
 
 // Device buffer owned by a context or reconstruction.
 struct DevBuf {
@@ -62,8 +61,6 @@ struct gf_ctx {
   int2* d_rowmap = nullptr;
   int* d_rowplane = nullptr;  // per padded row: FpArgs::rowplane
   int4* d_runs = nullptr;
-  float* d_gtab = nullptr;
-  float gtab_sigma = -1.f;
   // scratch of the operator entry points, allocated on first use
   int64_t launches = 0;  // kernels launched by this context
   // Bumped whenever a launch parameter that a captured graph holds changes
@@ -89,7 +86,6 @@ struct gf_ctx {
     return alloc(n * sizeof(T), reinterpret_cast<void**>(p));
   }
   gf_status ensure_scratch();
-  gf_status ensure_gtab(float sigma3d);
   gf::FpArgs fp_args(int subset, const float* img_zfast) const;
   gf::BpArgs bp_args(int subset, const gf::BpFrame& f, int storage) const;
   gf::BpTile bp_tile(int storage) const { return gf::bp_tile(plan, bp_warps, storage == GF_STORE_F32 ? 4 : 2); }

@@ -135,7 +135,7 @@ cudaError_t launch_cylinder(const DevGeom& g, float val, void* out, cudaStream_t
 // store: element type of the image arguments (0 FP32, 1 FP16, 2 BF16)
 cudaError_t launch_max_nonneg(const DevGeom& g, const void* img, float* d_max, cudaStream_t st, int store = 0);
 cudaError_t launch_bilateral(const DevGeom& g, const void* in, const void* ref, const float* d_max_ref,
-                             float max_ref, int r, float sigmai, const float* gtab, float* out, cudaStream_t st,
+                             float max_ref, int r, float sigma3d, float sigmai, float* out, cudaStream_t st,
                              int store = 0);
 cudaError_t launch_blend(const DevGeom& g, void* img2, const float* filt, cudaStream_t st, int store = 0);
 

@@ -134,7 +134,7 @@ gf_status gf_recon::subiteration(int t, int s) {
     // GFIRST.cu:512-524: r=4, sigma3D=0.75, sigmaI=0.025, max_ref over the doubles image
     stage_begin(GF_STAGE_BILATERAL);
     GF_LAUNCH(c, launch_max_nonneg(c->dg, img[0], d_max, st, store(0)));
-    GF_LAUNCH(c, launch_bilateral(c->dg, img[1], img[0], d_max, 0.f, 4, 0.025f, c->d_gtab, filt, st, store(0)));
+    GF_LAUNCH(c, launch_bilateral(c->dg, img[1], img[0], d_max, 0.f, 4, 0.75f, 0.025f, filt, st, store(0)));
     GF_LAUNCH(c, launch_blend(c->dg, img[1], filt, st, store(1)));
     stage_end();
   }
@@ -287,7 +287,6 @@ gf_status gf_recon_create(gf_ctx* c, const gf_recon_params* prm, gf_recon** out)
     ALLOC(r->dbg[1], pl.all_elems());
     ALLOC(r->filt, pl.nvoxp);
     ALLOC(r->d_max, 1);
-    if ((st = c->ensure_gtab(0.75f)) != GF_OK) return fail(st);
   }
   if (prm->mode == 3) {
     ALLOC(r->proj_t, pl.ndata);
