@@ -31,13 +31,18 @@
 // a run costs 2 (ZR + 1) / ZR four-byte loads; the lanes of a 4x8 tile at a
 // bin stride of 4 words modulo 8 conflict about 1.2-fold (16x2 tiles 1.6, 32x1
 // 2.1).  Preclinical subset (128x128x159 voxels, 53 segments, 10 angles),
-// FP32: 535 us per launch against 1120 us for one warp per column in the
-// per-view form, 700 against 1280 us per voxel; FP16 ratios 568 against 998 us
-// (the conversions).  Measured on the way: four-warp CTAs 594 us (twice the
+// FP32: 523 us per launch against 1120 us for one warp per column in the
+// per-view form, 638 against 1280 us per voxel (704 with each voxel's fraction
+// computed); FP16 ratios 561 against 998 us (the conversions).  With 2 % random
+// gaps, per voxel, FP32 at the reference geometry: 4.32 ms for a full
+// projection against 6.12 (4.64 with tiny weights looked for in every lane).
+// Measured on the way: four-warp CTAs 594 us (twice the
 // copies), the warps of a CTA along z instead of across columns 785 us (the
 // end runs wait for the middle ones), the lanes' weights from a table in
 // shared memory instead of recomputed 550 us, groups of half as many views
 // 640 us (barriers).
+#include <type_traits>
+
 #include "gf_kernels.h"
 
 namespace gf {
@@ -267,14 +272,20 @@ __global__ void __launch_bounds__(256) bp_tile_kernel(const BpArgs a) {
     const float be = __fsub_rn(t, ft);
     const bool edge = !FAST && be > 0.9999f;  // such a lane: every voxel is evaluated on its own
     auto frac = [&](int i) {
-      if constexpr (FAST) return be;
       const float fiz = (float)(z0 + i);
       const float zb = __fsub_rn(__fadd_rn(__fadd_rn(fiz, t), 0.5f), 0.5f);
       return __fsub_rn(zb, fiz + ft);
     };
+    // Those sums round the fraction of t to the spacing of floats at n = iz +
+    // floor(t), as long as n and n + 1 lie in one power-of-two interval: where
+    // the whole run does, its first voxel's fraction is every voxel's (five
+    // additions a voxel less in most runs).
+    const int n0 = z0 + (int)ft;
+    const float bf = FAST ? be : frac(0);
+    const bool flat = FAST || __all_sync(kAll, n0 > 0 && __clz(n0) == __clz(n0 + ZR));
 
-    if (__all_sync(kAll, (unsigned)(j0 - pad) < (unsigned)h.y && !edge)) {
-      // every voxel of every lane between two rows of the segment, no dead bin
+    // every voxel of every lane between two rows of the segment, no dead bin
+    auto interior = [&](auto one) {
       float S[ZR + 1];
       const float2 al2 = make_float2(al, al);
 #pragma unroll
@@ -287,7 +298,7 @@ __global__ void __launch_bounds__(256) bp_tile_kernel(const BpArgs a) {
       int sign = 0;
 #pragma unroll
       for (int i = 0; i < ZR; i++) {
-        S[i] = lerp_rn(S[i], S[i + 1], frac(i));
+        S[i] = lerp_rn(S[i], S[i + 1], one ? bf : frac(i));
         sign |= __float_as_int(S[i]);
       }
       if (!__any_sync(kAll, sign < 0)) {
@@ -304,6 +315,12 @@ __global__ void __launch_bounds__(256) bp_tile_kernel(const BpArgs a) {
 #pragma unroll
         for (int i = 0; i < ZR; i++) count_sample(num[i], den[i], S[i]);
       }
+    };
+    if (__all_sync(kAll, (unsigned)(j0 - pad) < (unsigned)h.y && !edge)) {
+      if (flat)
+        interior(std::true_type());
+      else
+        interior(std::false_type());
       return;
     }
 
@@ -328,28 +345,36 @@ __global__ void __launch_bounds__(256) bp_tile_kernel(const BpArgs a) {
     // The mask can only be positive with a masked corner where every masked
     // corner weighs next to nothing; those voxels (and the edge lanes') are
     // evaluated one by one.  Per voxel, the fractions are within 5e-5 of be.
+    // Most warps have no lane with both such a weight and a masked row.
     const float wa = 1.f - al, wl = 1.f - be;
-    auto unless = [](float wgt) { return wgt <= kTinyWeight ? kAll : 0u; };
-    unsigned cand = (ma | unless(wa * wl)) & ((ma >> 1) | unless(wa * be)) & (mb | unless(al * wl)) &
-                    ((mb >> 1) | unless(al * be)) & range & ~ok;
-    if (edge) cand = has ? bits(0, last) : 0u;
-    if (!__any_sync(kAll, (ok | cand) != 0u)) return;
+    const bool tiny = ok != range && (fminf(wa, al) * fminf(wl, be) <= kTinyWeight || edge);
     // The lanes' ranges differ by little: most runs at an edge have stretches
     // that no lane needs.
     constexpr int ZG = ZR % 5 == 0 ? 5 : 4;
     const unsigned some = __reduce_or_sync(kAll, ok);
+    auto masked = [&](auto one) {
 #pragma unroll
-    for (int i0 = 0; i0 < ZR; i0 += ZG) {
-      if (!(some & (((1u << ZG) - 1u) << i0))) continue;  // whole warp
-      float S = radial(i0);
+      for (int i0 = 0; i0 < ZR; i0 += ZG) {
+        if (!(some & (((1u << ZG) - 1u) << i0))) continue;  // whole warp
+        float S = radial(i0);
 #pragma unroll
-      for (int i = i0; i < i0 + ZG; i++) {
-        const float Sn = radial(i + 1);
-        const float v = lerp_rn(S, Sn, frac(i));
-        S = Sn;
-        count_sample(num[i], den[i], v, ok, 1u << i);
+        for (int i = i0; i < i0 + ZG; i++) {
+          const float Sn = radial(i + 1);
+          const float v = lerp_rn(S, Sn, one ? bf : frac(i));
+          S = Sn;
+          count_sample(num[i], den[i], v, ok, 1u << i);
+        }
       }
-    }
+    };
+    if (flat)
+      masked(std::true_type());
+    else
+      masked(std::false_type());
+    if (!__any_sync(kAll, tiny)) return;
+    auto unless = [](float wgt) { return wgt <= kTinyWeight ? kAll : 0u; };
+    unsigned cand = (ma | unless(wa * wl)) & ((ma >> 1) | unless(wa * be)) & (mb | unless(al * wl)) &
+                    ((mb >> 1) | unless(al * be)) & range & ~ok;
+    if (edge) cand = has ? bits(0, last) : 0u;
     const unsigned any = __reduce_or_sync(kAll, cand);
     if (any) {
       const float zlo = (float)h2.z, zhi = (float)(g.nzs - h2.z);

@@ -121,3 +121,26 @@ def test_staged_views_fit_their_slots(geo, warps, zr, eb):
                 assert (lo >= ra)[has].all() and (hi <= rb)[has].all()
                 q = (blk - 32 * wb + j0)[has]
                 assert q.min() >= 0 and (q // 32).max() + 1 < sh["mw"]
+
+
+@pytest.mark.parametrize("zr", [4, 12, 20])
+def test_run_fraction_is_every_voxels(zr):
+    """Where a run's n = iz + floor(t) stays in one power-of-two interval (and
+    n + zr too), the per-voxel form's fraction is that of its first voxel."""
+    rs = np.random.RandomState(zr)
+    t = (rs.uniform(-60, 60, 500000) * 10.0 ** rs.uniform(-7, 0, 500000)).astype(F)
+    t[:1000] = 0
+    z0 = rs.randint(0, 500, t.size)
+    ft = np.floor(t)
+    n0 = z0 + ft.astype(np.int64)
+    one = (n0 > 0) & (np.frexp(np.maximum(n0, 1))[1] == np.frexp(np.maximum(n0 + zr, 1))[1])
+    one &= ~((t - ft).astype(F) > F(0.9999))  # such lanes go voxel by voxel
+
+    def fraction(i):
+        fiz = (z0 + i).astype(F)
+        return ((fiz + t + F(0.5)) - F(0.5)) - (fiz + ft)
+
+    first = fraction(0)
+    assert first.dtype == F and one.sum() > 100000
+    for i in range(1, zr):
+        assert np.array_equal(fraction(i)[one], first[one])
