@@ -248,47 +248,67 @@ cudaError_t launch_pairs_from_file(const DevGeom& g, const int2* rowmap, int sub
 }
 
 // Ratio for the VLOR triples (GFIRST.cu:415-430 with val_dato = datos_v*RES,
-// GFIRST.cu:397, 421) of one subset, as ratios or, with cal, (ratio, mask) pairs.
+// GFIRST.cu:397, 421) of one subset, as ratios or, with cal, (ratio, mask)
+// pairs; projection and data come in 32x32 tiles as above.  Bound: HBM latency
+// and bytes.  One element a thread, with both file arrays read along rows (a
+// sector per element), took 36 us at 21 angles x 147 bins x 1293 planes, tiles 29.
 template <int STORE, bool PAIRS>
-__global__ void ratio_gather_kernel(const DevGeom g, const int2* __restrict__ rowmap, int subset,
-                                    const float* __restrict__ proj_full, const float* __restrict__ datos_v,
-                                    const float2* __restrict__ dbg_t, const float* __restrict__ cal,
-                                    void* __restrict__ out, size_t n) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int p = (int)(i % g.PS);
-  const size_t q = i / g.PS;
-  const int r = (int)(q % g.nrad), tl = (int)(q / g.nrad);
+__global__ void __launch_bounds__(256) ratio_gather_kernel(const DevGeom g, const int2* __restrict__ rowmap, int subset,
+                                                           const float* __restrict__ proj_full,
+                                                           const float* __restrict__ datos_v,
+                                                           const float2* __restrict__ dbg_t,
+                                                           const float* __restrict__ cal, void* __restrict__ out) {
+  __shared__ float tp[32][33], td[32][33];
+  const int r0 = blockIdx.x * 32, p0 = blockIdx.y * 32, tl = blockIdx.z;
   const int theta = subset_angle(g, subset, tl);
-  int seg, plane;
-  float v = -1000.f, mask = -1000.f;
-  const int2 m = rowmap[p];
-  if (resolve_row(g, m, &seg, &plane)) {
-    const size_t lor = file_lor(g, seg, plane, theta, r);
-    // the edge row's own element for segment 0's pad rows
-    const int prow = (m.y >= 0) ? p : (m.y == -1 ? p + 1 : p - 1);
-    const size_t e = i - p + prow;
-    const float data = __fmul_rn(datos_v[lor], (float)g.res);
-    v = ratio_rule(proj_full[lor], data, dbg_t[e].y);
-    if (PAIRS) mask = cal[e];
+  const int tx = threadIdx.x, ty = threadIdx.y;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const int p = p0 + ty + 8 * k, r = r0 + tx;
+    float proj = 0.f, data = 0.f;
+    int seg, plane;
+    if (r < g.nrad && resolve_row(g, rowmap[p], &seg, &plane)) {
+      const size_t lor = file_lor(g, seg, plane, theta, r);
+      proj = proj_full[lor];
+      data = datos_v[lor];
+    }
+    tp[ty + 8 * k][tx] = proj;
+    td[ty + 8 * k][tx] = data;
   }
-  if constexpr (PAIRS) {
-    using P = typename PairT<STORE>::type;
-    static_cast<P*>(out)[i] = pair_from<P>(make_float2(v, mask));
-  } else {
-    using T = typename ElemT<STORE>::type;
-    static_cast<T*>(out)[i] = elem_from<T>(v);
+  __syncthreads();
+  const int p = p0 + tx;
+  const int2 m = rowmap[p];
+  int seg, plane;
+  const bool row = resolve_row(g, m, &seg, &plane);
+  // the edge row's own element for segment 0's pad rows
+  const int prow = (m.y >= 0) ? p : (m.y == -1 ? p + 1 : p - 1);
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const int r = r0 + ty + 8 * k;
+    if (r >= g.nrad) break;
+    const size_t at = ((size_t)tl * g.nrad + r) * g.PS;
+    float v = -1000.f, mask = -1000.f;
+    if (row) {
+      v = ratio_rule(tp[tx][ty + 8 * k], __fmul_rn(td[tx][ty + 8 * k], (float)g.res), dbg_t[at + prow].y);
+      if (PAIRS) mask = cal[at + prow];
+    }
+    if constexpr (PAIRS) {
+      using P = typename PairT<STORE>::type;
+      static_cast<P*>(out)[at + p] = pair_from<P>(make_float2(v, mask));
+    } else {
+      using T = typename ElemT<STORE>::type;
+      static_cast<T*>(out)[at + p] = elem_from<T>(v);
+    }
   }
 }
 
 cudaError_t launch_ratio_gather(const DevGeom& g, const int2* rowmap, int subset, int na, const float* proj_full,
                                 const float* datos_v, const float2* dbg_t, const float* cal, void* out, int storage,
                                 cudaStream_t st) {
-  const size_t n = (size_t)na * g.nrad * g.PS;
-  const unsigned nb = (unsigned)((n + 255) / 256);
+  const dim3 grid((g.nrad + 31) / 32, g.PS / 32, na), block(32, 8);
   switch (storage * 2 + (cal ? 1 : 0)) {
 #define GF_RG(S, P) \
-  case S * 2 + P: ratio_gather_kernel<S, P><<<nb, 256, 0, st>>>(g, rowmap, subset, proj_full, datos_v, dbg_t, cal, out, n); break;
+  case S * 2 + P: ratio_gather_kernel<S, P><<<grid, block, 0, st>>>(g, rowmap, subset, proj_full, datos_v, dbg_t, cal, out); break;
     GF_RG(0, 0) GF_RG(0, 1) GF_RG(1, 0) GF_RG(1, 1) GF_RG(2, 0) GF_RG(2, 1)
 #undef GF_RG
     default: return cudaErrorInvalidValue;
@@ -420,46 +440,56 @@ cudaError_t launch_vlor_sort(const DevGeom& g, const int32_t* ev, long long nev,
   return cub::DeviceRadixSort::SortKeys(temp, temp_bytes, keys_tmp, keys, (int)(2 * nev), 0, 64, st);
 }
 
-// pass 1, over events: both shares of each event, share[2e + end]
-__global__ void vlor_shares_kernel(const int32_t* __restrict__ ev, long long nev, long long ndata,
-                                   const float* __restrict__ proj, const float* __restrict__ bl, float* share) {
-  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nev) return;
-  long long i1, i2;
-  if (!vlor_bins(ev, e, ndata, &i1, &i2)) return;  // its keys are kNoKey: never read
-  const float valor = __fadd_rn(bl[i1], bl[i2]);
-  const float s1 = proj[i1], s2 = proj[i2];
-  const float s = __fadd_rn(s1, s2);
-  const float s_inv = (s > 0.01f) ? (float)__drcp_rn((double)s) : 0.f;
-  share[2 * e] = __fmul_rn(__fmul_rn(s1, s_inv), valor);
-  share[2 * e + 1] = __fmul_rn(__fmul_rn(s2, s_inv), valor);
-}
-
-// pass 2, over the sorted ends: the first end of each bin adds the bin's
-// shares in event order
-__global__ void vlor_split_sorted_kernel(const unsigned long long* __restrict__ keys, long long n,
-                                         const float* __restrict__ share, float* out) {
+// Both passes walk the sorted ends, so the two file-sized arrays are read in
+// address order; what is random stays in an array of 16 bytes an event.  One
+// pass over the events for their shares, reading projection and weight of two
+// random bins each, and one over the sorted ends for the shares took 61 + 30 us
+// for a million events in 32 M bins; these take 41 + 31.
+// pass 1: projection and weight of each end's bin, ends[2e + end]
+__global__ void __launch_bounds__(256) vlor_ends_kernel(const unsigned long long* __restrict__ keys, long long n,
+                                                        const float* __restrict__ proj, const float* __restrict__ bl,
+                                                        float2* __restrict__ ends) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const unsigned long long k = keys[i];
   if (k == kNoKey) return;
+  ends[k & 0xffffffffull] = make_float2(proj[k >> 32], bl[k >> 32]);
+}
+
+// pass 2: the first end of each bin adds the bin's shares in event order
+__global__ void __launch_bounds__(256) vlor_split_sorted_kernel(const unsigned long long* __restrict__ keys,
+                                                                long long n, const float4* __restrict__ events,
+                                                                float* out) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  unsigned long long k = keys[i];
+  if (k == kNoKey) return;
   const unsigned long long bin = k >> 32;
   if (i > 0 && (keys[i - 1] >> 32) == bin) return;  // not the first share of its bin
   float sum = out[bin];  // the shares are added to out, as the reference adds them to SINOG_VLOR
-  for (long long j = i; j < n && (keys[j] >> 32) == bin; j++) sum = __fadd_rn(sum, share[keys[j] & 0xffffffffull]);
+  for (long long j = i;;) {
+    const float4 e = events[(k & 0xffffffffull) >> 1];  // (projection, weight) of its two ends
+    const float valor = __fadd_rn(e.y, e.w);
+    const float s = __fadd_rn(e.x, e.z);
+    const float s_inv = (s > 0.01f) ? (float)__drcp_rn((double)s) : 0.f;
+    sum = __fadd_rn(sum, __fmul_rn(__fmul_rn((k & 1) ? e.z : e.x, s_inv), valor));
+    if (++j >= n) break;
+    k = keys[j];
+    if ((k >> 32) != bin) break;
+  }
   out[bin] = sum;
 }
 
 cudaError_t launch_vlor_split_sorted(const DevGeom& g, const unsigned long long* keys, long long nev,
-                                     const int32_t* ev, const float* proj, const float* blankt, float* share,
-                                     float* out, cudaStream_t st) {
+                                     const float* proj, const float* blankt, float2* ends, float* out,
+                                     cudaStream_t st) {
   if (nev <= 0) return cudaSuccess;
-  const long long ndata = (long long)g.P * g.nang * g.nrad;
-  vlor_shares_kernel<<<(unsigned)((nev + 255) / 256), 256, 0, st>>>(ev, nev, ndata, proj, blankt, share);
+  const long long n = 2 * nev;
+  const unsigned nb = (unsigned)((n + 255) / 256);
+  vlor_ends_kernel<<<nb, 256, 0, st>>>(keys, n, proj, blankt, ends);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  const long long n = 2 * nev;
-  vlor_split_sorted_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(keys, n, share, out);
+  vlor_split_sorted_kernel<<<nb, 256, 0, st>>>(keys, n, reinterpret_cast<const float4*>(ends), out);
   return cudaGetLastError();
 }
 
