@@ -6,7 +6,9 @@
 // and tile shapes form fused groups of up to kMaxFrames, whatever their
 // subset counts, whose sub-iterations run every stage as one launch over the
 // frames that have that subset (fused_subiteration); every other frame is a
-// unit of its own.
+// unit of its own.  Where the back projector runs one warp per column, frames of
+// a group with the same subset count and equal normalization masks (the frames of
+// one scanner and normalization) back-project two per warp.
 //
 // One iteration of every unit is captured once: a fork event on the batch's
 // origin stream, each unit's kernels on the stream of its first frame (a
@@ -30,7 +32,7 @@ using namespace gf;
 struct gf_batch {
   std::vector<gf_recon*> frames;
   int device = 0;
-  int fused = 0;  // gf_batch_set_fused: 0 off, 1 or 2 groups (1: gf_batch_groups counts pairs of equal masks)
+  int fused = 0;  // gf_batch_set_fused: 0 off, 1 groups (frames of equal masks in pairs), 2 groups
   std::vector<std::vector<int>> units;  // frame indices: a fused group, or one frame
   // per unit and member: its class (the first member with the same subset
   // count and an equal normalization mask), or -1
@@ -42,7 +44,14 @@ struct gf_batch {
   cudaGraphExec_t exec = nullptr;
   cudaGraph_t graph = nullptr;
   std::vector<std::pair<int64_t, int64_t>> cap_gen;  // (context, reconstruction) generations at capture
+  std::vector<int64_t> cap_norm;                     // gf_recon::norm_gen when cls was last right
 };
+
+static std::vector<int64_t> norm_gens(const gf_batch* b) {
+  std::vector<int64_t> v;
+  for (const gf_recon* r : b->frames) v.push_back(r->norm_gen);
+  return v;
+}
 
 static bool stale(const gf_batch* b) {
   for (size_t i = 0; i < b->frames.size(); i++) {
@@ -80,14 +89,17 @@ static void make_units(gf_batch* b) {
 
 // The frames of a fused group that have the same subset count and equal
 // normalization masks (every subset, in that count's layout), compared on the
-// device after the frames' queued work (their loads) has finished.
-static gf_status check_masks(gf_batch* b) {
+// device after the frames' queued work (their loads) has finished.  Where the
+// back projector runs one warp per column such frames share it two by two;
+// to_run: only these are compared.
+static gf_status check_masks(gf_batch* b, bool to_run) {
   b->cls.assign(b->units.size(), {});
   for (size_t k = 0; k < b->units.size(); k++) {
     const auto& u = b->units[k];
     b->cls[k].assign(u.size(), -1);
     if (b->fused != 1 || u.size() < 2) continue;
     if (b->frames[u[0]]->ctx->bp_form != GF_BP_PER_VIEW) continue;
+    if (to_run && !b->frames[u[0]]->cal) continue;  // column tiles take each frame on its own
     for (size_t j = 0; j < u.size(); j++) {
       const gf_recon* r = b->frames[u[j]];
       b->cls[k][j] = (int)j;  // a class of its own unless an earlier leader matches
@@ -132,9 +144,14 @@ static gf_status unit_iteration(gf_batch* b, size_t k) {
   for (int i : u) smax = std::max(smax, b->frames[i]->ctx->plan.nsub);
   for (int s = 0; s < smax; s++) {
     std::vector<gf_recon*> G;
-    for (int i : u)
-      if (b->frames[i]->ctx->plan.nsub > s) G.push_back(b->frames[i]);
-    GF_TRY(fused_subiteration(G.data(), (int)G.size(), st));
+    std::vector<int> C;
+    for (size_t j = 0; j < u.size(); j++) {
+      gf_recon* r = b->frames[u[j]];
+      if (r->ctx->plan.nsub <= s) continue;
+      G.push_back(r);
+      C.push_back(b->cls[k][j]);
+    }
+    GF_TRY(fused_subiteration(G.data(), (int)G.size(), C.data(), st));
   }
   return GF_OK;
 }
@@ -198,13 +215,16 @@ gf_status gf_batch_set_fused(gf_batch* b, int32_t fused) {
 gf_status gf_batch_groups(gf_batch* b, int32_t* ngroups, int32_t* largest, int32_t* paired) {
   if (!b) return set_error(GF_ERR_ARG, "null batch");
   GF_CK(cudaSetDevice(b->device));
-  GF_TRY(check_masks(b));
+  const auto captured = b->cls;
+  GF_TRY(check_masks(b, false));
+  const auto cls = b->cls;
+  if (b->exec) b->cls = captured;
   int n = 0, big = 0, pairs = 0;
   for (size_t k = 0; k < b->units.size(); k++) {
     n++;
     big = std::max(big, (int)b->units[k].size());
     // pairs of the first step, where every member takes part
-    const std::vector<int>& c = b->cls[k];
+    const std::vector<int>& c = cls[k];
     for (size_t j = 0; j < c.size(); j++)
       if (c[j] == (int)j) pairs += (int)std::count(c.begin(), c.end(), (int)j) / 2;
   }
@@ -224,6 +244,7 @@ static gf_status capture(gf_batch* b) {
   make_units(b);
   // the frames' streams must be idle before they join the capture
   for (gf_recon* r : b->frames) GF_CK(cudaStreamSynchronize(r->ctx->stream));
+  GF_TRY(check_masks(b, true));
   std::vector<bool> prof(b->frames.size());
   std::vector<gf_ctx*> ctxs;  // each context once: frames may share one
   std::vector<int64_t> l0;
@@ -280,6 +301,7 @@ static gf_status capture(gf_batch* b) {
   GF_CK(cudaGraphInstantiate(&b->exec, g, 0));
   b->cap_gen.clear();
   for (gf_recon* r : b->frames) b->cap_gen.emplace_back(r->ctx->gen, r->gen);
+  b->cap_norm = norm_gens(b);
   // capturing advanced every frame's host cursor by one iteration, but the
   // captured work has not run: the first replay below is that iteration
   for (gf_recon* r : b->frames) {
@@ -296,6 +318,7 @@ gf_status gf_batch_iterate(gf_batch* b, int32_t n, int32_t use_graph) {
   GF_CK(cudaSetDevice(b->device));
   if (!use_graph) {
     make_units(b);
+    GF_TRY(check_masks(b, true));
     for (int it = 0; it < n; it++) {
       for (size_t ku = 0; ku < b->units.size(); ku++) {
         const std::vector<int>& u = b->units[ku];
@@ -323,6 +346,16 @@ gf_status gf_batch_iterate(gf_batch* b, int32_t n, int32_t use_graph) {
     // a replay still queued on the origin stream may use the old graph
     GF_CK(cudaStreamSynchronize(b->origin));
     drop_graph(b);
+  }
+  if (b->exec && b->cap_norm != norm_gens(b)) {
+    // masks loaded since the capture: its pairs may no longer share one
+    const auto cls = b->cls;
+    GF_TRY(check_masks(b, true));
+    b->cap_norm = norm_gens(b);
+    if (cls != b->cls) {
+      GF_CK(cudaStreamSynchronize(b->origin));
+      drop_graph(b);
+    }
   }
   if (!b->exec) GF_TRY(capture(b));
   // the frames' own streams may hold work queued outside the graph

@@ -159,6 +159,8 @@ __global__ void __launch_bounds__(256) bp_tile_kernel(const BpArgs a) {
   // this lane's column (a tile that reaches past the image repeats its last columns)
   const int ix = cx0 + (w >> 1) * kTileX + lane % kTileX, iy = cy0 + (w & 1) * kTileY + lane / kTileX;
   const bool mine = ix < g.res && iy < g.res;
+  // a warp whose whole tile is past the image only stages
+  const bool inside = cx0 + (w >> 1) * kTileX < g.res && cy0 + (w & 1) * kTileY < g.res;
   const float xv = __fsub_rn((float)min(ix, g.res - 1), g.resm), yv = __fsub_rn((float)min(iy, g.res - 1), g.resm);
   // a corner of the CTA's columns: every coordinate is monotone in x and in y,
   // rounding included, so its extremes over the columns are at the corners
@@ -424,7 +426,8 @@ __global__ void __launch_bounds__(256) bp_tile_kernel(const BpArgs a) {
     if (v0 + nw + w < nviews) stage(s, tl, slot_of(buf ^ 1, w));
     cp_async_commit();
     const int n = min(nw, nviews - v0);
-    for (int u = 0; u < n; u++) view(slot_of(buf, u));
+    if (inside)
+      for (int u = 0; u < n; u++) view(slot_of(buf, u));
     buf ^= 1;
   }
 
@@ -452,9 +455,8 @@ __global__ void __launch_bounds__(256) bp_tile_kernel(const BpArgs a) {
     }
 }
 
-template <class T>
+template <int ZR, class T>
 static cudaError_t launch_tiles_t(const BpArgs& a, int warps, cudaStream_t st) {
-  constexpr int ZR = kTileRun;
   auto k = a.fast ? bp_tile_kernel<ZR, T, true> : bp_tile_kernel<ZR, T, false>;
   const size_t smem = (size_t)32 * a.na + (size_t)2 * warps * a.slot_bytes;
   if (smem > 48 * 1024) {
@@ -467,18 +469,26 @@ static cudaError_t launch_tiles_t(const BpArgs& a, int warps, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+template <int ZR>
+static cudaError_t launch_tiles_z(const BpArgs& a, int warps, cudaStream_t st) {
+  switch (a.storage) {
+    case 0: return launch_tiles_t<ZR, float>(a, warps, st);
+    case 1: return launch_tiles_t<ZR, __half>(a, warps, st);
+    case 2: return launch_tiles_t<ZR, __nv_bfloat16>(a, warps, st);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
 cudaError_t launch_bp_tiles(const BpArgs& in, const BpTile& tile, cudaStream_t st) {
-  if (tile.zr != kTileRun) return cudaErrorInvalidValue;
   BpArgs a = in;
   a.nsw = (a.g.nseg + 31) / 32;
   a.rs = tile.rs;
   a.mw = tile.mw;
   a.rows_at = tile.rows_at;
   a.slot_bytes = tile.slot_bytes;
-  switch (a.storage) {
-    case 0: return launch_tiles_t<float>(a, tile.warps, st);
-    case 1: return launch_tiles_t<__half>(a, tile.warps, st);
-    case 2: return launch_tiles_t<__nv_bfloat16>(a, tile.warps, st);
+  switch (tile.zr) {
+    case kTileRun: return launch_tiles_z<kTileRun>(a, tile.warps, st);
+    case kShortRun: return launch_tiles_z<kShortRun>(a, tile.warps, st);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -88,7 +88,9 @@ struct gf_ctx {
   gf_status ensure_scratch();
   gf::FpArgs fp_args(int subset, const float* img_zfast) const;
   gf::BpArgs bp_args(int subset, const gf::BpFrame& f, int storage) const;
-  gf::BpTile bp_tile(int storage) const { return gf::bp_tile(plan, bp_warps, storage == GF_STORE_F32 ? 4 : 2); }
+  gf::BpTile bp_tile(int storage, int frames = 1) const {
+    return gf::bp_tile(plan, bp_warps, storage == GF_STORE_F32 ? 4 : 2, frames);
+  }
 };
 
 struct gf_recon {
@@ -150,6 +152,7 @@ struct gf_recon {
   // Bumped when a load changes what an iteration's launches capture (the
   // mode-3 event count or event buffers); gf_batch recaptures on a change.
   int64_t gen = 0;
+  int64_t norm_gen = 0;  // loads of a normalization mask
 
   // stage profiling
   struct StageEv {
@@ -186,5 +189,7 @@ bool fusable(const gf_recon* a, const gf_recon* b);
 // them, on stream st (the group's: its first member's, which need not take
 // part in every step) with the first frame's tables.  Advances every frame's
 // cursor.
-gf_status fused_subiteration(gf_recon* const* G, int nfr, cudaStream_t st);
+// cls: frames with the same class >= 0 (same subset count and normalization
+// mask; per-view form, one warp per column) back-project two per warp.
+gf_status fused_subiteration(gf_recon* const* G, int nfr, const int* cls, cudaStream_t st);
 }  // namespace gf

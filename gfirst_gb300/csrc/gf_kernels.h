@@ -83,7 +83,9 @@ struct BpArgs {
   int pad_lo, rbuf;
   BpFrame fr[kMaxFrames];
 };
-cudaError_t launch_bp(const BpArgs& a, const BpTile& tile, cudaStream_t st);
+// pairs: one warp per column and two frames, a.fr[2p] and a.fr[2p + 1], of equal
+// masks (per-view form, tile.zr = 0).
+cudaError_t launch_bp(const BpArgs& a, const BpTile& tile, cudaStream_t st, bool pairs = false);
 cudaError_t launch_bp_tiles(const BpArgs& a, const BpTile& tile, cudaStream_t st);  // gf_bp_tile.cu
 // Lets kernel k use up to the device's opt-in shared memory per block.  Every
 // call sets the same value, so host threads that launch one kernel with

@@ -16,6 +16,8 @@ static int seg_zmin(const Geom& g, int idz) {
   return idz == 0 ? 0 : (std::abs(idz) - 1) * g.span + (g.span / 2 + 1);
 }
 
+static bool tiles_pay(const Plan& p);
+
 bool make_plan(const Geom& g, int nsub, Plan* out, std::string* err) {
   auto fail = [&](const char* m) {
     if (err) *err = m;
@@ -76,6 +78,8 @@ bool make_plan(const Geom& g, int nsub, Plan* out, std::string* err) {
   p.sub_off.assign(nsub + 1, 0);
   for (int s = 0; s < nsub; s++) p.sub_off[s + 1] = p.sub_off[s] + p.sub_elems(s);
   p.amax = *std::max_element(p.sub_nang.begin(), p.sub_nang.end());
+  p.pads = bp_fast_pads(p);
+  p.tiles = tiles_pay(p);
   *out = std::move(p);
   return true;
 }
@@ -153,16 +157,17 @@ BpPads bp_fast_pads(const Plan& p) {
 }
 
 // The tile shape of a plan, whether or not it is used.
-static BpTile tile_shape(const Plan& p, int warps, int elem_bytes) {
+static BpTile tile_shape(const Plan& p, int warps, int elem_bytes, int zr) {
   BpTile t;
   t.warps = warps;
   // Slices of a run: longer runs share the radial interpolation of a row and a
   // view's set-up among more voxels, shorter ones waste less at the ends of a
   // segment and make more CTAs.  12 / 16 slices, us a launch: 535 / 523 (128 x
   // 128 x 159 voxels, 53 segments, 10 angles, per-view form), 701 / 705 (per
-  // voxel), 332 / 322 (15 segments, 21 angles), 201 / 226 (96^3), 102 / 116 (72^3).
+  // voxel), 332 / 322 (15 segments, 21 angles), 201 / 226 (96^3).  8 slices:
+  // see run_length.
   const int cx = kTileX * (warps / 2), cy = kTileY * 2;
-  t.zr = kTileRun;
+  t.zr = zr;
   // the CTA's columns are at most `diag` voxels apart, and so are their
   // in-plane coordinates rotated to any angle
   const double diag = std::hypot((double)(cx - 1), (double)(cy - 1));
@@ -184,23 +189,40 @@ static BpTile tile_shape(const Plan& p, int warps, int elem_bytes) {
   return t;
 }
 
-// Tiles where their 8-warp CTAs (16 x 16 columns, one run) give about every SM
-// one; below, a view's latency shows and one warp per column is faster.
-// Columns / tiles, us a launch, by the number of CTAs: 54 / 95 at 48 CTAs (64 x
-// 64 x 32), 68 / 89 at 96 (64^3), 171 / 202 at 126 (48 x 48 x 159), 153 / 102
-// at 150 (72^3), 134 / 104 at 192 (128 x 128 x 32), 350 / 197 at 288 (96^3),
-// 1120 / 535 at 896 (128 x 128 x 159).
-bool bp_uses_tiles(const Plan& p) {
-  const BpTile t = tile_shape(p, 8, 4);  // the largest of its slots
-  if (2ll * t.warps * t.slot_bytes + 32ll * p.amax > 160 * 1024) return false;
-  const int b = (p.g.res + 15) / 16;
-  return b * b * ((p.g.nzs + kTileRun - 1) / kTileRun) >= 150;
+// Warps of 12-slice runs over the image (its columns in 4x8 tiles), in CTAs of 8.
+static long long run_ctas(const Plan& p) {
+  return (long long)((p.g.res + kTileX - 1) / kTileX) * ((p.g.res + kTileY - 1) / kTileY) *
+         ((p.g.nzs + kTileRun - 1) / kTileRun) / 8;
 }
 
-BpTile bp_tile(const Plan& p, int warps, int elem_bytes) {
-  BpTile t = tile_shape(p, warps, elem_bytes);
+// Tiles where their CTAs fill the SMs with warps that hide a view's latency;
+// below, one warp per column is faster.  Fewer segments are fewer views for a
+// CTA's set-up, and need more CTAs; a single segment stays with columns.  Back
+// projection and the forward projection that feeds it, tiles against columns,
+// by run_ctas and segments, without gaps / with 2 % of the bins masked (per-view
+// form; per voxel within 0.1 above): 0.73 / 0.97 at 172 and 29 (90 x 90 x 54),
+// 0.91 / 1.22 at 243 and 19 (69 x 69 x 138), 0.66 / 0.90 at 250 and 35 (80 x 80 x
+// 110), 0.78 / 1.04 at 260 and 17 (82 x 82 x 99), 0.71 / 0.99 at 261 and 21 (75 x
+// 75 x 126), 0.76 / 0.95 at 272 and 5 (115 x 115 x 51), 0.69 / 0.91 at 276 and 53
+// (91 x 91 x 90), 0.75 / 0.95 at 333 and 11 (88 x 88 x 129), 0.62 / 0.79 at 372 and
+// 7 (124 x 124 x 69), 0.93 / 1.14 at 406 and 5 (97 x 97 x 117), 0.65 / 0.80 at 441
+// and 15 (110 x 110 x 101); 0.95 / 1.13 at 272 and 1 (88 x 88 x 98).
+static bool tiles_pay(const Plan& p) {
+  const BpTile t = tile_shape(p, 8, 4, kTileRun);  // the largest of its slots
+  if (2ll * t.warps * t.slot_bytes + 32ll * p.amax > 160 * 1024) return false;
+  return p.g.nseg > 1 && run_ctas(p) >= 245 + 9 * std::max(0, 20 - p.g.nseg);
+}
+
+// Runs of 8 slices while runs of 12 leave every SM fewer than two CTAs (three
+// fit).  12 / 8 slices, us a launch: 143 / 130 at 260 (82 x 82 x 99), 283 / 236
+// at 272 (115 x 115 x 51), 303 / 289 at 276 (91 x 91 x 90), 199 / 219 at 288
+// (96^3), 56 / 72 at 333 (88 x 88 x 129), 84 / 97 at 441 (110 x 110 x 101).
+static int run_length(const Plan& p, int frames) { return run_ctas(p) * frames < 285 ? kShortRun : kTileRun; }
+
+BpTile bp_tile(const Plan& p, int warps, int elem_bytes, int frames) {
+  BpTile t = tile_shape(p, warps, elem_bytes, run_length(p, frames));
   if (!bp_uses_tiles(p)) t.zr = 0;
-  t.pads = bp_fast_pads(p);
+  t.pads = p.pads;
   return t;
 }
 

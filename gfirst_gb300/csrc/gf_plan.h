@@ -37,6 +37,18 @@ struct Run {
   int seg, p0, n, pad;  // pad: bit0 = writes the row before, bit1 = after
 };
 
+// Staged-row buffer of the back projector's per-view form: each warp stages a
+// view's rows at offset pad_lo of a buffer of rbuf (corr, calib) pairs, the
+// rest held at the -1000 gap sentinel.  A lane chunk reads its two rows at
+// an offset fixed per view, so voxels outside the segment's plane range read
+// sentinels there (or the segment's own sentinel pad rows with weight >=
+// 1/2), which the gap rule skips as the range test would.  pad_lo and the
+// rows past the widest segment cover every row any issued lane chunk reads,
+// for every axial shift |t| <= |yrot| * |fz| the geometry allows.
+struct BpPads {
+  int pad_lo = 0, pad_hi = 0, rbuf = 0;
+};
+
 struct Plan {
   Geom g{};
   int P = 0, PP = 0, PS = 0, NZP = 0;
@@ -49,6 +61,8 @@ struct Plan {
   std::vector<int> sub_nang;     // angles per subset
   std::vector<int64_t> sub_off;  // element offset of subset s in an all-subset array
   int amax = 0;                  // most angles in one subset
+  BpPads pads;                   // bp_fast_pads
+  bool tiles = false;            // back projections run as column tiles (bp_uses_tiles)
   int64_t sub_elems(int s) const { return (int64_t)sub_nang[s] * g.nrad * PS; }
   int64_t all_elems() const { return (int64_t)g.nang * g.nrad * PS; }
 };
@@ -66,24 +80,14 @@ struct FpSchedule {
 bool make_fp_schedule(const Plan& p, int R, int lc, FpSchedule* out);
 int fp_default_R(const Plan& p);
 
-// Staged-row buffer of the back projector's per-view form: each warp stages a
-// view's rows at offset pad_lo of a buffer of rbuf (corr, calib) pairs, the
-// rest held at the -1000 gap sentinel.  A lane chunk reads its two rows at
-// an offset fixed per view, so voxels outside the segment's plane range read
-// sentinels there (or the segment's own sentinel pad rows with weight >=
-// 1/2), which the gap rule skips as the range test would.  pad_lo and the
-// rows past the widest segment cover every row any issued lane chunk reads,
-// for every axial shift |t| <= |yrot| * |fz| the geometry allows.
-struct BpPads {
-  int pad_lo = 0, pad_hi = 0, rbuf = 0;
-};
+// The staged-row buffer of a plan (Plan::pads holds it).
 BpPads bp_fast_pads(const Plan& p);
 
 // Shape of the back projector's work.  Column tiles (gf_bp_tile.cu): a warp owns
-// kTileX x kTileY columns and a run of zr = kTileRun slices, a CTA `warps` such
-// tiles (two in y) and one run.  zr = 0: one warp per column (gf_bp.cu), `warps`
+// kTileX x kTileY columns and a run of zr slices (kTileRun, or kShortRun where
+// that makes few CTAs), a CTA `warps` such tiles (two in y) and one run.  zr = 0: one warp per column (gf_bp.cu), `warps`
 // a block.
-constexpr int kTileX = 4, kTileY = 8, kTileRun = 12;
+constexpr int kTileX = 4, kTileY = 8, kTileRun = 12, kShortRun = 8;
 // Elements before a staged view's first row: a lane's run may start that far
 // before the segment's rows.
 constexpr int bp_pad_front(int zr, int elem_bytes) {
@@ -98,8 +102,9 @@ struct BpTile {
 };
 // Whether a plan's back projections run as column tiles: a property of the
 // plan alone, since the sinogram layouts of a reconstruction follow from it.
-bool bp_uses_tiles(const Plan& p);
-BpTile bp_tile(const Plan& p, int warps, int elem_bytes);
+inline bool bp_uses_tiles(const Plan& p) { return p.tiles; }
+// The shape for a launch over `frames` images of the plan.
+BpTile bp_tile(const Plan& p, int warps, int elem_bytes, int frames = 1);
 
 // Sinogram bin of (segment, plane, angle, radial), GFIRST.cu:175-176.
 inline int64_t lor_index(const Plan& p, int s, int iz0, int t, int r) {

@@ -166,10 +166,10 @@ bool fusable(const gf_recon* a, const gf_recon* b) {
   return a->p.mode == 1 && b->p.mode == 1 && a->loaded && b->loaded && x->device == y->device && same_geom &&
          a->p.storage == b->p.storage && a->p.image_storage == b->p.image_storage && a->p.psf_fw == b->p.psf_fw &&
          a->p.psf_bw == b->p.psf_bw && x->bp_form == y->bp_form && x->bp_warps == y->bp_warps &&
-         x->fps.R == y->fps.R && x->fps.lc == y->fps.lc;
+         x->fps.R == y->fps.R && x->fps.lc == y->fps.lc && bp_uses_tiles(x->plan) == bp_uses_tiles(y->plan);
 }
 
-gf_status fused_subiteration(gf_recon* const* G, int nfr, cudaStream_t st) {
+gf_status fused_subiteration(gf_recon* const* G, int nfr, const int* cls, cudaStream_t st) {
   if (nfr < 1 || nfr > kMaxFrames) return set_error(GF_ERR_ARG, "fused group size out of range");
   gf_recon* r0 = G[0];
   gf_ctx* c = r0->ctx;
@@ -195,7 +195,8 @@ gf_status fused_subiteration(gf_recon* const* G, int nfr, cudaStream_t st) {
   }
   GF_LAUNCH(c, launch_fp(a, c->fps, st));
   // the back projector keeps the subset a launch constant: one launch per
-  // subset count among the frames
+  // subset count among the frames; one warp per column also takes frames of
+  // one class two by two
   std::vector<bool> done(nfr, false);
   for (int k0 = 0; k0 < nfr; k0++) {
     if (done[k0]) continue;
@@ -204,13 +205,28 @@ gf_status fused_subiteration(gf_recon* const* G, int nfr, cudaStream_t st) {
     b.g.nsub = pl.nsub;
     b.na = pl.sub_nang[s];
     b.ratio = 1;
-    b.nfr = 0;
+    std::vector<int> pairs, singles;
     for (int k = k0; k < nfr; k++) {
       if (done[k] || G[k]->ctx->plan.nsub != pl.nsub) continue;
       done[k] = true;
-      b.fr[b.nfr++] = G[k]->bp_frame(s);
+      int j = -1;
+      if (b.fast && G[k]->cal && cls && cls[k] >= 0)
+        for (int m = k + 1; m < nfr && j < 0; m++)
+          if (!done[m] && cls[m] == cls[k]) j = m;
+      if (j >= 0) {
+        done[j] = true;
+        pairs.push_back(k);
+        pairs.push_back(j);
+      } else {
+        singles.push_back(k);
+      }
     }
-    GF_LAUNCH(c, launch_bp(b, c->bp_tile(r0->p.storage), st));
+    for (const auto* v : {&pairs, &singles}) {
+      if (v->empty()) continue;
+      b.nfr = 0;
+      for (int k : *v) b.fr[b.nfr++] = G[k]->bp_frame(s);
+      GF_LAUNCH(c, launch_bp(b, c->bp_tile(r0->p.storage, b.nfr), st, v == &pairs));
+    }
   }
   ImgFrames u{};
   for (int k = 0; k < nfr; k++) u.fr[k] = ImgFrame{G[k]->ratio, nullptr, G[k]->img[0]};
@@ -380,6 +396,7 @@ static gf_status load_impl(gf_recon* r, const float* h_image, const float* h_dsi
   if ((s = ck(cudaEventRecord(r->ev_staged, cs), "record staging")) != GF_OK) return done(s);
   if ((s = ck(cudaStreamWaitEvent(st, r->ev_staged, 0), "wait upload")) != GF_OK) return done(s);
   if ((s = ck(launch_build_dbg(c->dg, c->d_rowmap, s2, r->dbg[0], st), "build data")) != GF_OK) return done(s);
+  r->norm_gen++;
   if (r->cal) {
     if ((s = ck(launch_build_cal(c->dg, c->d_rowmap, r->proj_ref, sn, r->cal, st), "build mask")) != GF_OK) return done(s);
   } else {

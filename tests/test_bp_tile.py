@@ -59,7 +59,7 @@ GEOS = [(128, 159, 128, 160, 3, 53, 1.6, 165.7758, 100.0), (128, 159, 147, 168, 
 
 
 @pytest.mark.parametrize("geo", GEOS, ids=lambda g: f"{g[0]}x{g[1]}_{g[2]}x{g[3]}")
-@pytest.mark.parametrize("warps,zr,eb", [(8, 12, 4), (8, 12, 2), (4, 12, 4), (4, 12, 2)])
+@pytest.mark.parametrize("warps,zr,eb", [(8, 12, 4), (8, 12, 2), (4, 12, 4), (4, 12, 2), (8, 8, 4), (8, 8, 2), (4, 8, 4), (4, 8, 2)])
 def test_staged_views_fit_their_slots(geo, warps, zr, eb):
     res, nzs, nrad, nang, span, nseg, pitch, diam, fov = geo
     sh = tile_shape(geo, warps, zr, eb)
@@ -123,7 +123,7 @@ def test_staged_views_fit_their_slots(geo, warps, zr, eb):
                 assert q.min() >= 0 and (q // 32).max() + 1 < sh["mw"]
 
 
-@pytest.mark.parametrize("zr", [4, 12, 20])
+@pytest.mark.parametrize("zr", [8, 12, 20])
 def test_run_fraction_is_every_voxels(zr):
     """Where a run's n = iz + floor(t) stays in one power-of-two interval (and
     n + zr too), the per-voxel form's fraction is that of its first voxel."""

@@ -24,6 +24,8 @@ GEOS = [
     (131, 27, 90, 5, 5, 3, 2.1, 150.0, 101.0),  # wide and flat: 81 blocks, 3 runs, the last of 3 slices
     (66, 256, 61, 4, 7, 35, 1.6, 90.0, 54.0),  # the deepest image, segments past the 32nd
     (66, 160, 61, 3, 1, 71, 1.6, 90.0, 54.0),  # segments past the 64th
+    (130, 61, 90, 5, 3, 11, 1.8, 150.0, 101.0),  # runs of 12, remainders in x, y and z
+    (102, 66, 81, 6, 1, 21, 1.6, 100.0, 72.0),   # runs of 8, remainders in x, y and z
 ]
 
 
@@ -112,7 +114,7 @@ def test_tiles_match_oracle(gf, geo, gaps):  # noqa: F811
 
 
 def test_masks_of_other_values_match_oracle(gf):  # noqa: F811
-    geo = GEOS[0]
+    geo = GEOS[-1]
     o = gfo.Oracle(geo)
     ctx = gf.Context(gf.Geometry(*geo), nsub=2)
     corr, calib = ratio_and_mask(o, geo, 6, 0.02)
@@ -129,7 +131,7 @@ def test_masks_of_other_values_match_oracle(gf):  # noqa: F811
 
 
 def test_infinities_and_nan_match_oracle(gf):  # noqa: F811
-    geo = GEOS[0]
+    geo = GEOS[-1]
     o = gfo.Oracle(geo)
     ctx = gf.Context(gf.Geometry(*geo), nsub=2)
     corr, calib = ratio_and_mask(o, geo, 9, 0.02)
@@ -144,9 +146,9 @@ def test_infinities_and_nan_match_oracle(gf):  # noqa: F811
 
 @pytest.mark.parametrize("mode,storage,tol", [(1, "f32", IMG_TOL), (3, "f32", IMG_TOL), (1, "f16", IMG_TOL),
                                               (1, "bf16", 10 * IMG_TOL)])
-def test_reconstruction_over_tiles_matches_oracle(gf, mode, storage, tol):  # noqa: F811
+@pytest.mark.parametrize("geo", [(72, 72, 72, 8, 3, 5, 1.6, 95.48, 57.6), GEOS[-1]], ids=["72", "102"])
+def test_reconstruction_over_tiles_matches_oracle(gf, geo, mode, storage, tol):  # noqa: F811
     """16-bit ratios round by 2^-11 (2^-8 in BF16) per sample, 2 subsets of one iteration."""
-    geo = (72, 72, 72, 8, 3, 5, 1.6, 95.48, 57.6)
     o = gfo.Oracle(geo)
     rs = np.random.RandomState(11)
     nd = o.ndata

@@ -14,7 +14,8 @@ from test_gpu_parity import IMG_TOL, gf, rel  # noqa: F401
 pytestmark = pytest.mark.gpu
 
 SMALL = (40, 33, 37, 9, 3, 7, 1.6, 53.0, 32.0)    # (ratio, mask) pairs
-TILES = (73, 75, 70, 7, 3, 9, 1.6, 95.8, 58.4)    # ratios and mask bits
+TILES = (73, 75, 70, 7, 3, 9, 1.6, 95.8, 58.4)
+BITS = (102, 66, 81, 6, 1, 21, 1.6, 100.0, 72.0)  # ratios and mask bits
 
 
 @pytest.mark.parametrize("n", [1, 2, 127, 128, 129, 4097])
@@ -32,7 +33,7 @@ def test_split_matches_oracle(gf, n):  # noqa: F811
     assert np.array_equal(out.download(), o.vlor_split(ev, proj, bl))
 
 
-@pytest.mark.parametrize("geo", [SMALL, TILES], ids=["pairs", "tiles"])
+@pytest.mark.parametrize("geo", [SMALL, TILES, BITS], ids=["pairs", "wide", "bits"])
 def test_triples_match_oracle(gf, geo):  # noqa: F811
     o = gfo.Oracle(geo)
     rs = np.random.RandomState(8)
