@@ -363,9 +363,10 @@ class Batch:
 
     def set_fused(self, fused: bool = True, pairs: bool = True) -> None:
         """Fused groups: frames that match (any subset counts) run each stage
-        as one launch; with pairs, groups() counts the frame pairs of one subset
-        count and equal normalization (gf_batch_set_fused 1, else 2;
-        fused=False: 0)."""
+        as one launch; with pairs, frames of one subset count and equal
+        normalization count as pairs and share the back projector's work where
+        it runs one warp per column (gf_batch_set_fused 1, else 2; fused=False:
+        0)."""
         _ck(lib().gf_batch_set_fused(self.h, 0 if not fused else (1 if pairs else 2)))
 
     def groups(self) -> tuple:

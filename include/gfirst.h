@@ -284,12 +284,12 @@ gf_status gf_batch_synchronize(gf_batch* b);
  * frames that have a subset s, each at its own subset s; the forward PSF,
  * projection + ratio and update are one kernel launch over those frames and
  * the back projection one launch per subset count among them, each frame
- * keeping its own data and results (the same as alone, bit for bit).  fused =
- * 1 and 2 run the same launches; with 1, gf_batch_groups also compares the
- * normalization masks of a group's frames (on the device) and counts the pairs
- * of frames that share subset count and mask under the per-view form.  Other
- * frames run on their own.  0 turns fusing off.  Takes effect at the next
- * iterate. */
+ * keeping its own data and results (the same as alone, bit for bit).  With
+ * fused = 1, frames of a group with the same subset count and equal
+ * normalization masks (checked on the device), back projector in the per-view
+ * form, count as pairs, and back-project two per warp where it runs one warp
+ * per column; fused = 2 keeps one frame per warp.  Other frames run on their
+ * own.  0 turns fusing off.  Takes effect at the next iterate. */
 gf_status gf_batch_set_fused(gf_batch* b, int32_t fused);
 /* Units the batch runs (fused groups and single frames), the size of the
  * largest group and the pairs of frames of equal subset count and mask (fused
