@@ -404,6 +404,7 @@ def run_gpu(args) -> int:
     alg = algorithmic_bytes(P, ndata, nvox)
     peak, peak_src = peaks()
     traffic = committed_traffic()
+    traffic.update(traffic.get("tiles", {}))  # the layout that this plan runs
     dom = max(("fp", "bp"), key=lambda k: stage.get(k, {}).get("total_ms", 0.0))
     roof = {}
     for k in ("fp", "bp"):
