@@ -25,9 +25,9 @@
 // views read one bit per row.  Samples with a masked corner of a tiny weight
 // are evaluated one by one with the reference's expression.
 //
-// Bound: instruction issue (71 % of peak while SMs are busy, 419 M warp
+// Bound: instruction issue (76 % of peak while SMs are busy, 463 M warp
 // instructions at the preclinical subset against 777 M for one warp per
-// column; shared-memory wavefronts 48 % of peak, DRAM 1 %).  Per voxel and lane
+// column; data-pipe wavefronts 53 % of peak, DRAM 1 %).  Per voxel and lane
 // a run costs 2 (ZR + 1) / ZR four-byte loads; the lanes of a 4x8 tile at a
 // bin stride of 4 words modulo 8 conflict about 1.2-fold (16x2 tiles 1.6, 32x1
 // 2.1).  Preclinical subset (128x128x159 voxels, 53 segments, 10 angles),
