@@ -7,6 +7,7 @@
 // 508-539) and layout conversions.  All of these are HBM-bound except the
 // bilateral filter; they keep the reference's operation order with explicit
 // round-to-nearest arithmetic so their results equal the reference's.
+#include <cfloat>
 #include <cmath>
 
 #include "gf_kernels.h"
@@ -371,12 +372,17 @@ __device__ __forceinline__ float ex2(float x) {
 // a thread owns one slice (its lane) of BL_N columns along x, so the BL_N + 2 R
 // values of a window row are loaded once for all of them.  Voxels with a
 // coordinate below R give 0 (the reference's unsigned window start wraps and
-// its loops run zero times); past the far sides the staged reference is
-// infinite, which makes the weight 0.  A tap's weight is exp of the intensity
-// and the x distance together, one ex2 of a fused multiply-add; the y and z
-// part of the spatial weight scales a row's two sums.  FP32 throughout, where
-// the reference evaluates its exponentials in double: 3e-7 from 64 bits on
-// 128x128x159 voxels (9e-7 with a weight of two factors).
+// its loops run zero times).  A tap's weight is exp of the intensity and the x
+// distance together, one ex2 of a fused multiply-add; the y and z part of the
+// spatial weight scales a row's two sums.  FP32 throughout, where the reference
+// evaluates its exponentials in double: 3e-7 from 64 bits on 128x128x159 voxels
+// (9e-7 with a weight of two factors).
+//
+// Past the far sides the staged reference is infinite, which makes the weight 0
+// where the intensity scale is a normal number (bl_ordinary).  Other scales -- no
+// range term (an infinite sigmai or max_ref), a product of two ordinary factors
+// that under- or overflows, 0, NaN -- take the GENERAL kernel: the two factors one
+// after the other, taps past the far sides left out by their coordinates.
 //
 // Bound: the 729 exponentials a voxel (16 a clock and SM: 377 us for 128x128x159
 // voxels), with instruction issue 86 % busy beside them.  gf_bilateral on
@@ -391,12 +397,21 @@ struct BlTaps {
   float lx[BL_H + 1];  // log2 of the spatial weight at distance 0..BL_H along an axis
 };
 
-template <class T, int R>
+// exp(-(d / max_ref)^2 / ci) = 2^-(d k)^2 with k = root_log2e_ci / max_ref
+__host__ __device__ __forceinline__ float bl_scale(float max_ref, float root_log2e_ci) {
+  return (1.0f / max_ref) * root_log2e_ci;
+}
+__host__ __device__ __forceinline__ bool bl_ordinary(float k) { return fabsf(k) >= FLT_MIN && fabsf(k) <= FLT_MAX; }
+
+// With max_ref on the device the GENERAL kernel follows the other one and ends at
+// once where the scale is ordinary (as a test in one kernel it cost 2 %).
+template <class T, int R, bool GENERAL>
 __global__ void __launch_bounds__(512, 2) bilateral_kernel(const DevGeom g, const T* __restrict__ in,
                                                            const T* __restrict__ ref,
                                                            const float* __restrict__ d_max_ref, float max_ref_host,
                                                            float root_log2e_ci, const BlTaps taps,
                                                            float* __restrict__ out) {
+  if (GENERAL && d_max_ref && bl_ordinary(bl_scale(*d_max_ref, root_log2e_ci))) return;
   extern __shared__ float bl_smem[];
   float* Sr = bl_smem;
   float* Si = bl_smem + BL_W * BL_W * BL_Z;
@@ -420,7 +435,8 @@ __global__ void __launch_bounds__(512, 2) bilateral_kernel(const DevGeom g, cons
   const int y = y0 + ty, z = z0 + lane;
   if (y >= RES || x0 + tx >= RES) return;  // whole warp
   const float max_ref = d_max_ref ? *d_max_ref : max_ref_host;
-  const float k = (1.0f / max_ref) * root_log2e_ci;  // exp(-(d / max_ref)^2 / ci) = 2^-(d k)^2
+  const float k = bl_scale(max_ref, root_log2e_ci);
+  const float rinv = 1.0f / max_ref;
   const int at = ((ty + BL_H) * BL_W + tx + BL_H) * BL_Z + lane + BL_H;
   float ref0[BL_N], norm[BL_N], sum[BL_N];
 #pragma unroll
@@ -433,6 +449,7 @@ __global__ void __launch_bounds__(512, 2) bilateral_kernel(const DevGeom g, cons
 #pragma unroll 1
     for (int dy = -R; dy <= R; dy++) {
       const int row = at + dy * BL_W * BL_Z + dz;
+      const bool in_yz = y + dy < RES && z + dz < NZS;
       float r[BL_N + 2 * R], v[BL_N + 2 * R];
 #pragma unroll
       for (int i = 0; i < BL_N + 2 * R; i++) {
@@ -445,8 +462,9 @@ __global__ void __launch_bounds__(512, 2) bilateral_kernel(const DevGeom g, cons
         float rn = 0.f, rs = 0.f;
 #pragma unroll
         for (int i = 0; i <= 2 * R; i++) {
-          const float d = (r[n + i] - ref0[n]) * k;
-          const float w = ex2(__fmaf_rn(-d, d, taps.lx[i < R ? R - i : i - R]));
+          const float d = GENERAL ? (r[n + i] - ref0[n]) * rinv * root_log2e_ci : (r[n + i] - ref0[n]) * k;
+          float w = ex2(__fmaf_rn(-d, d, taps.lx[i < R ? R - i : i - R]));
+          if (GENERAL && !(in_yz && x0 + tx + n + i - R < RES)) w = 0.f;
           rn += w;
           rs = __fmaf_rn(w, v[n + i], rs);
         }
@@ -465,16 +483,28 @@ __global__ void __launch_bounds__(512, 2) bilateral_kernel(const DevGeom g, cons
   }
 }
 
-template <class T, int R>
-static cudaError_t launch_bilateral_r(const DevGeom& g, const void* in, const void* ref, const float* d_max_ref,
+template <class T, int R, bool GENERAL>
+static cudaError_t launch_bilateral_g(const DevGeom& g, const void* in, const void* ref, const float* d_max_ref,
                                       float max_ref, float root, const BlTaps& taps, float* out, cudaStream_t st) {
-  auto k = bilateral_kernel<T, R>;
+  auto k = bilateral_kernel<T, R, GENERAL>;
   cudaError_t e = allow_max_smem(k);
   if (e != cudaSuccess) return e;
   const dim3 grid((g.res + BL_T - 1) / BL_T, (g.res + BL_T - 1) / BL_T, g.nzp / 32);
   k<<<grid, 512, kBlSmem, st>>>(g, static_cast<const T*>(in), static_cast<const T*>(ref), d_max_ref, max_ref, root, taps,
                                 out);
   return cudaGetLastError();
+}
+
+template <class T, int R>
+static cudaError_t launch_bilateral_r(const DevGeom& g, const void* in, const void* ref, const float* d_max_ref,
+                                      float max_ref, float root, const BlTaps& taps, float* out, cudaStream_t st) {
+  const bool ordinary = bl_ordinary(bl_scale(max_ref, root));  // of a max_ref known here
+  cudaError_t e = cudaSuccess;
+  if (d_max_ref || ordinary)
+    e = launch_bilateral_g<T, R, false>(g, in, ref, d_max_ref, max_ref, root, taps, out, st);
+  if (e == cudaSuccess && (d_max_ref || !ordinary))
+    e = launch_bilateral_g<T, R, true>(g, in, ref, d_max_ref, max_ref, root, taps, out, st);
+  return e;
 }
 
 template <class T>
