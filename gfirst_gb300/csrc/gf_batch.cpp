@@ -44,7 +44,8 @@ struct gf_batch {
   cudaGraphExec_t exec = nullptr;
   cudaGraph_t graph = nullptr;
   std::vector<std::pair<int64_t, int64_t>> cap_gen;  // (context, reconstruction) generations at capture
-  std::vector<int64_t> cap_norm;                     // gf_recon::norm_gen when cls was last right
+  std::vector<std::vector<int>> cap_cls;             // classes at capture: the graph's pairs
+  std::vector<int64_t> cap_norm;                     // gf_recon::norm_gen when cap_cls was last right
 };
 
 static std::vector<int64_t> norm_gens(const gf_batch* b) {
@@ -92,19 +93,19 @@ static void make_units(gf_batch* b) {
 // device after the frames' queued work (their loads) has finished.  Where the
 // back projector runs one warp per column such frames share it two by two;
 // to_run: only these are compared.
-static gf_status check_masks(gf_batch* b, bool to_run) {
-  b->cls.assign(b->units.size(), {});
+static gf_status check_masks(const gf_batch* b, bool to_run, std::vector<std::vector<int>>* out) {
+  std::vector<std::vector<int>> cls(b->units.size());
   for (size_t k = 0; k < b->units.size(); k++) {
     const auto& u = b->units[k];
-    b->cls[k].assign(u.size(), -1);
+    cls[k].assign(u.size(), -1);
     if (b->fused != 1 || u.size() < 2) continue;
     if (b->frames[u[0]]->ctx->bp_form != GF_BP_PER_VIEW) continue;
     if (to_run && !b->frames[u[0]]->cal) continue;  // column tiles take each frame on its own
     for (size_t j = 0; j < u.size(); j++) {
       const gf_recon* r = b->frames[u[j]];
-      b->cls[k][j] = (int)j;  // a class of its own unless an earlier leader matches
+      cls[k][j] = (int)j;  // a class of its own unless an earlier leader matches
       for (size_t i = 0; i < j; i++) {
-        if (b->cls[k][i] != (int)i) continue;  // not a class leader
+        if (cls[k][i] != (int)i) continue;  // not a class leader
         const gf_recon* l = b->frames[u[i]];
         if (l->ctx->plan.nsub != r->ctx->plan.nsub) continue;
         bool same = false;
@@ -122,12 +123,13 @@ static gf_status check_masks(gf_batch* b, bool to_run) {
           same = flag == 0;
         }
         if (same) {
-          b->cls[k][j] = (int)i;
+          cls[k][j] = (int)i;
           break;
         }
       }
     }
   }
+  *out = std::move(cls);
   return GF_OK;
 }
 
@@ -215,10 +217,8 @@ gf_status gf_batch_set_fused(gf_batch* b, int32_t fused) {
 gf_status gf_batch_groups(gf_batch* b, int32_t* ngroups, int32_t* largest, int32_t* paired) {
   if (!b) return set_error(GF_ERR_ARG, "null batch");
   GF_CK(cudaSetDevice(b->device));
-  const auto captured = b->cls;
-  GF_TRY(check_masks(b, false));
-  const auto cls = b->cls;
-  if (b->exec) b->cls = captured;
+  std::vector<std::vector<int>> cls;
+  GF_TRY(check_masks(b, false, &cls));
   int n = 0, big = 0, pairs = 0;
   for (size_t k = 0; k < b->units.size(); k++) {
     n++;
@@ -244,7 +244,7 @@ static gf_status capture(gf_batch* b) {
   make_units(b);
   // the frames' streams must be idle before they join the capture
   for (gf_recon* r : b->frames) GF_CK(cudaStreamSynchronize(r->ctx->stream));
-  GF_TRY(check_masks(b, true));
+  GF_TRY(check_masks(b, true, &b->cls));
   std::vector<bool> prof(b->frames.size());
   std::vector<gf_ctx*> ctxs;  // each context once: frames may share one
   std::vector<int64_t> l0;
@@ -301,6 +301,7 @@ static gf_status capture(gf_batch* b) {
   GF_CK(cudaGraphInstantiate(&b->exec, g, 0));
   b->cap_gen.clear();
   for (gf_recon* r : b->frames) b->cap_gen.emplace_back(r->ctx->gen, r->gen);
+  b->cap_cls = b->cls;
   b->cap_norm = norm_gens(b);
   // capturing advanced every frame's host cursor by one iteration, but the
   // captured work has not run: the first replay below is that iteration
@@ -318,7 +319,7 @@ gf_status gf_batch_iterate(gf_batch* b, int32_t n, int32_t use_graph) {
   GF_CK(cudaSetDevice(b->device));
   if (!use_graph) {
     make_units(b);
-    GF_TRY(check_masks(b, true));
+    GF_TRY(check_masks(b, true, &b->cls));
     for (int it = 0; it < n; it++) {
       for (size_t ku = 0; ku < b->units.size(); ku++) {
         const std::vector<int>& u = b->units[ku];
@@ -349,10 +350,9 @@ gf_status gf_batch_iterate(gf_batch* b, int32_t n, int32_t use_graph) {
   }
   if (b->exec && b->cap_norm != norm_gens(b)) {
     // masks loaded since the capture: its pairs may no longer share one
-    const auto cls = b->cls;
-    GF_TRY(check_masks(b, true));
+    GF_TRY(check_masks(b, true, &b->cls));
     b->cap_norm = norm_gens(b);
-    if (cls != b->cls) {
+    if (b->cls != b->cap_cls) {
       GF_CK(cudaStreamSynchronize(b->origin));
       drop_graph(b);
     }
