@@ -236,6 +236,7 @@ gf_status gf_create(const gf_geometry* g, int32_t nsubsets, int32_t device, gf_c
     cudaGetLastError();
   }
   gf_ctx* c = new gf_ctx();
+  plan.pads = bp_fast_pads(plan);
   c->bp_warps = bp_uses_tiles(plan) ? 8 : 4;
   c->plan = std::move(plan);
   c->fps = std::move(fps);

@@ -78,7 +78,6 @@ bool make_plan(const Geom& g, int nsub, Plan* out, std::string* err) {
   p.sub_off.assign(nsub + 1, 0);
   for (int s = 0; s < nsub; s++) p.sub_off[s + 1] = p.sub_off[s] + p.sub_elems(s);
   p.amax = *std::max_element(p.sub_nang.begin(), p.sub_nang.end());
-  p.pads = bp_fast_pads(p);
   p.tiles = tiles_pay(p);
   *out = std::move(p);
   return true;

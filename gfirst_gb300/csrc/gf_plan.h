@@ -61,7 +61,7 @@ struct Plan {
   std::vector<int> sub_nang;     // angles per subset
   std::vector<int64_t> sub_off;  // element offset of subset s in an all-subset array
   int amax = 0;                  // most angles in one subset
-  BpPads pads;                   // bp_fast_pads
+  BpPads pads;                   // bp_fast_pads; set by gf_create alone: its loop takes longer than all else here
   bool tiles = false;            // back projections run as column tiles (bp_uses_tiles)
   int64_t sub_elems(int s) const { return (int64_t)sub_nang[s] * g.nrad * PS; }
   int64_t all_elems() const { return (int64_t)g.nang * g.nrad * PS; }
@@ -80,7 +80,7 @@ struct FpSchedule {
 bool make_fp_schedule(const Plan& p, int R, int lc, FpSchedule* out);
 int fp_default_R(const Plan& p);
 
-// The staged-row buffer of a plan (Plan::pads holds it).
+// The staged-row buffer of a plan (a context's Plan::pads holds it).
 BpPads bp_fast_pads(const Plan& p);
 
 // Shape of the back projector's work.  Column tiles (gf_bp_tile.cu): a warp owns
