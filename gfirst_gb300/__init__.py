@@ -134,6 +134,13 @@ def bp_staged_rows(g: Geometry) -> dict:
     return {"pad_lo": lo.value, "pad_hi": hi.value, "rbuf": rb.value}
 
 
+def bp_run(g: Geometry, nsub: int = 1, images: int = 1) -> int:
+    """Slices of a run where back projections go over column tiles, 0 for one warp per column (gf_bp_run)."""
+    n = ctypes.c_int32()
+    _ck(lib().gf_bp_run(ctypes.byref(g.c()), nsub, images, ctypes.byref(n)))
+    return n.value
+
+
 def lor_index(g: Geometry, seg: int, iz0: int, theta: int, ird: int) -> int:
     out = ctypes.c_int64()
     _ck(lib().gf_lor_index(ctypes.byref(g.c()), seg, iz0, theta, ird, ctypes.byref(out)))

@@ -137,6 +137,17 @@ gf_status gf_bp_staged_rows(const gf_geometry* g, int32_t* pad_lo, int32_t* pad_
   return GF_OK;
 }
 
+gf_status gf_bp_run(const gf_geometry* g, int32_t nsubsets, int32_t images, int32_t* slices) {
+  Geom geo;
+  if (!to_geom(g, &geo) || !slices) return set_error(GF_ERR_ARG, "null argument");
+  if (images < 1) return set_error(GF_ERR_ARG, "images must be positive");
+  Plan p;
+  std::string err;
+  if (!make_plan(geo, nsubsets, &p, &err)) return set_error(GF_ERR_GEOMETRY, err);
+  *slices = bp_tile(p, 8, 4, images).zr;
+  return GF_OK;
+}
+
 gf_status gf_kernel_launches(const gf_ctx* c, int64_t* n) {
   if (!c || !n) return set_error(GF_ERR_ARG, "null argument");
   *n = c->launches;

@@ -194,28 +194,43 @@ static long long run_ctas(const Plan& p) {
          ((p.g.nzs + kTileRun - 1) / kTileRun) / 8;
 }
 
-// Tiles where their CTAs fill the SMs with warps that hide a view's latency;
-// below, one warp per column is faster.  Fewer segments are fewer views for a
-// CTA's set-up, and need more CTAs; a single segment stays with columns.  Back
-// projection and the forward projection that feeds it, tiles against columns,
-// by run_ctas and segments, without gaps / with 2 % of the bins masked (per-view
-// form; per voxel within 0.1 above): 0.73 / 0.97 at 172 and 29 (90 x 90 x 54),
-// 0.91 / 1.22 at 243 and 19 (69 x 69 x 138), 0.66 / 0.90 at 250 and 35 (80 x 80 x
-// 110), 0.78 / 1.04 at 260 and 17 (82 x 82 x 99), 0.71 / 0.99 at 261 and 21 (75 x
-// 75 x 126), 0.76 / 0.95 at 272 and 5 (115 x 115 x 51), 0.69 / 0.91 at 276 and 53
-// (91 x 91 x 90), 0.75 / 0.95 at 333 and 11 (88 x 88 x 129), 0.62 / 0.79 at 372 and
-// 7 (124 x 124 x 69), 0.93 / 1.14 at 406 and 5 (97 x 97 x 117), 0.65 / 0.80 at 441
-// and 15 (110 x 110 x 101); 0.95 / 1.13 at 272 and 1 (88 x 88 x 98).
+// Tiles where their CTAs fill the SMs with warps that hide a view's latency and
+// enough of each CTA is image; elsewhere one warp per column.  Fewer segments are
+// fewer views for a CTA's set-up, and need more CTAs; a single segment stays with
+// columns.  The masked path is what decides: without masked bins tiles are the
+// faster far below the line, with 2 % of the bins masked they are not.
+// Back projection and the forward projection that feeds it, tiles against columns,
+// FP32, over 390 geometries of 48 to 128 columns, 24 to 159 slices and 1 to 53
+// segments: the 102 that run tiles take 0.56 to 0.89 of the columns' time without
+// masked bins (mean 0.69 per view, 0.74 per voxel) and 0.73 to 1.07 with 2 % (0.89,
+// 0.95).  The second condition is for CTAs that reach far past the image: without it
+// 1.12 / 1.20 (per view / per voxel, masked bins) at 69 x 69 x 147 and 25 segments,
+// 1.14 / 1.12 at 97 x 97 x 117 and 5, 1.05 / 1.13 at 117 x 117 x 102 and 3, 0.99 /
+// 1.13 at 98 x 98 x 86 and 31.  It leaves to columns a few that gain without masked
+// bins (97 x 97 x 117: 0.93; 98 x 98 x 86: 0.80), and the first one more (90 x 90 x
+// 54, 29 segments: 0.73, 0.97 with; 115 x 115 x 51, 5: 0.76, 0.95), because their
+// neighbours lose as much with them (84 x 84 x 54, 15: 1.24 per voxel).
 static bool tiles_pay(const Plan& p) {
   const BpTile t = tile_shape(p, 8, 4, kTileRun);  // the largest of its slots
   if (2ll * t.warps * t.slot_bytes + 32ll * p.amax > 160 * 1024) return false;
-  return p.g.nseg > 1 && run_ctas(p) >= 245 + 9 * std::max(0, 20 - p.g.nseg);
+  const int nseg = p.g.nseg;
+  if (nseg < 2 || run_ctas(p) < 245 + 9 * std::max(0, 20 - nseg)) return false;
+  constexpr int side = 16;  // columns of an 8-warp CTA, each way
+  const long long across = (p.g.res + side - 1) / side, along = (p.g.nzs + kTileRun - 1) / kTileRun;
+  const double launched = (double)(across * across * along);
+  const double useful = (double)p.g.res * p.g.res * p.g.nzs / (side * side * kTileRun);  // CTAs full of image
+  const double share = useful / launched;
+  return useful * share * share >= 130 + 40 * std::max(0, 8 - nseg);
 }
 
-// Runs of 8 slices while runs of 12 leave every SM fewer than two CTAs (three
-// fit).  12 / 8 slices, us a launch: 143 / 130 at 260 (82 x 82 x 99), 283 / 236
-// at 272 (115 x 115 x 51), 303 / 289 at 276 (91 x 91 x 90), 199 / 219 at 288
-// (96^3), 56 / 72 at 333 (88 x 88 x 129), 84 / 97 at 441 (110 x 110 x 101).
+// Runs of 8 slices while runs of 12 make few CTAs; one image alone, since two
+// frames of any plan with tiles have enough.  8 / 12 slices, per view and per
+// voxel without masked bins, by run_ctas: 1.01 / 0.93 at 250 (80 x 80 x 110), 0.91 /
+// 0.90 at 252 (93 x 93 x 83), 0.97 / 0.90 at 261 (74 x 74 x 130), 0.95 / 0.95 at 276
+// (91 x 91 x 90); then mixed, 1.10 at 288 (96^3, whole CTAs and runs), 1.00 / 0.97 at
+// 288 (95 x 95 x 85), 1.14 / 0.98 at 295 (104 x 104 x 82), 1.01 / 0.93 at 302 (88 x
+// 88 x 111), 0.97 / 0.90 at 330 (107 x 107 x 78); 12 ahead above: 1.18 / 1.05 at 332
+// (88 x 88 x 129), 1.20 / 1.01 at 346 (84 x 84 x 140).  The line lies below 96^3.
 static int run_length(const Plan& p, int frames) { return run_ctas(p) * frames < 285 ? kShortRun : kTileRun; }
 
 BpTile bp_tile(const Plan& p, int warps, int elem_bytes, int frames) {

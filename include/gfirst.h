@@ -105,6 +105,11 @@ gf_status gf_set_bp_form(gf_ctx* ctx, int32_t form);
  * (16 * angles per subset + 8 * rbuf) bytes. */
 gf_status gf_bp_staged_rows(const gf_geometry* g, int32_t* pad_lo, int32_t* pad_hi, int32_t* rbuf);
 
+/* How back projections of `images` images of a geometry run in one launch (no
+ * device work): column tiles over runs of *slices slices, or with *slices = 0 one
+ * warp per column. */
+gf_status gf_bp_run(const gf_geometry* g, int32_t nsubsets, int32_t images, int32_t* slices);
+
 /* Device memory helpers for callers without a CUDA runtime of their own. */
 gf_status gf_device_alloc(gf_ctx* ctx, size_t bytes, void** d_ptr);
 gf_status gf_device_free(gf_ctx* ctx, void* d_ptr);
