@@ -243,29 +243,45 @@ __global__ void __launch_bounds__(512, R == 9 && NB == 1 ? 2 : 1) fp_kernel(cons
     }
     __syncthreads();
     const size_t base = ((size_t)tl * g.nrad + ird) * g.PS;
-    for (int p = tid; p < g.PP; p += nt) {
-      // pad rows: segment 0's repeat its first and last plane, the others are gaps
-      const int pl = a.rowplane[p];
-      const int row = p == 0 ? 1 : (p == NZS + 1 ? NZS : p);
-      V proj{};
-      if (pl >= 0) proj = buf[pl];
+    // U rows of a thread at a time: their plane, then data loads are in flight together
+    constexpr int U = 4 / NB;
+    for (int p0 = tid; p0 < g.PP; p0 += U * nt) {
+      int pl[U];
 #pragma unroll
-      for (int b = 0; b < NB; b++) {
-        if (NB > 1 && ird + b >= g.nrad) break;  // whole block
-        const size_t o = base + (size_t)b * g.PS;
-        float corr = -1000.f, cal = -1000.f;
-        if (pl >= 0) {
-          const float2 db = F.dbg[o + row];
-          const float s = __fadd_rn(proj.v[b], db.y);
-          corr = (s >= 0.01f) ? __fdiv_rn(db.x, s) : -1000.f;
-          if (PAIRS) cal = F.cal[o + row];
+      for (int u = 0; u < U; u++) pl[u] = p0 + u * nt < g.PP ? a.rowplane[p0 + u * nt] : -1;
+      float2 db[U][NB];
+      float cal[U][NB];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        // pad rows: segment 0's repeat its first and last plane, the others are gaps
+        const int p = p0 + u * nt, row = p == 0 ? 1 : (p == NZS + 1 ? NZS : p);
+#pragma unroll
+        for (int b = 0; b < NB; b++) {
+          const bool in = pl[u] >= 0 && (NB == 1 || ird + b < g.nrad);
+          const size_t o = base + (size_t)b * g.PS + row;
+          db[u][b] = in ? F.dbg[o] : make_float2(0.f, 0.f);
+          cal[u][b] = PAIRS && in ? F.cal[o] : -1000.f;
         }
-        if constexpr (PAIRS) {
-          using P = typename PairT<STORE>::type;
-          static_cast<P*>(F.corr)[o + p] = pair_from<P>(make_float2(corr, cal));
-        } else {
-          using T = typename ElemT<STORE>::type;
-          static_cast<T*>(F.corr)[o + p] = elem_from<T>(corr);
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int p = p0 + u * nt;
+        if (p >= g.PP) break;
+        V proj{};
+        if (pl[u] >= 0) proj = buf[pl[u]];
+#pragma unroll
+        for (int b = 0; b < NB; b++) {
+          if (NB > 1 && ird + b >= g.nrad) break;  // whole block
+          const size_t o = base + (size_t)b * g.PS;
+          const float s = __fadd_rn(proj.v[b], db[u][b].y);
+          const float corr = pl[u] >= 0 && s >= 0.01f ? __fdiv_rn(db[u][b].x, s) : -1000.f;
+          if constexpr (PAIRS) {
+            using P = typename PairT<STORE>::type;
+            static_cast<P*>(F.corr)[o + p] = pair_from<P>(make_float2(corr, cal[u][b]));
+          } else {
+            using T = typename ElemT<STORE>::type;
+            static_cast<T*>(F.corr)[o + p] = elem_from<T>(corr);
+          }
         }
       }
     }
