@@ -141,6 +141,13 @@ def bp_run(g: Geometry, nsub: int = 1, images: int = 1) -> int:
     return n.value
 
 
+def fp_run(g: Geometry, nsub: int = 1, subset: int = 0) -> int:
+    """Radial bins that one block of a forward projection takes, 1 or 4 (gf_fp_run)."""
+    n = ctypes.c_int32()
+    _ck(lib().gf_fp_run(ctypes.byref(g.c()), nsub, subset, ctypes.byref(n)))
+    return n.value
+
+
 def lor_index(g: Geometry, seg: int, iz0: int, theta: int, ird: int) -> int:
     out = ctypes.c_int64()
     _ck(lib().gf_lor_index(ctypes.byref(g.c()), seg, iz0, theta, ird, ctypes.byref(out)))

@@ -148,6 +148,19 @@ gf_status gf_bp_run(const gf_geometry* g, int32_t nsubsets, int32_t images, int3
   return GF_OK;
 }
 
+gf_status gf_fp_run(const gf_geometry* g, int32_t nsubsets, int32_t subset, int32_t* bins) {
+  Geom geo;
+  if (!to_geom(g, &geo) || !bins) return set_error(GF_ERR_ARG, "null argument");
+  Plan p;
+  std::string err;
+  if (!make_plan(geo, nsubsets, &p, &err)) return set_error(GF_ERR_GEOMETRY, err);
+  if (subset < 0 || subset >= p.nsub) return set_error(GF_ERR_ARG, "subset out of range");
+  FpSchedule f;
+  if (!make_fp_schedule(p, fp_default_R(p), 32, &f)) return set_error(GF_ERR_GEOMETRY, "no forward-projector schedule fits");
+  *bins = fp_bins(f, geo.nseg, geo.nrad, p.sub_nang[subset]);
+  return GF_OK;
+}
+
 gf_status gf_kernel_launches(const gf_ctx* c, int64_t* n) {
   if (!c || !n) return set_error(GF_ERR_ARG, "null argument");
   *n = c->launches;

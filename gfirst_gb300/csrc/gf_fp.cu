@@ -235,53 +235,43 @@ __global__ void __launch_bounds__(512, R == 9 && NB == 1 ? 2 : 1) fp_kernel(cons
   if constexpr (RATIO) {
     // the projections in plane order through shared memory, so that the data
     // are read and the ratios written in whole lines
-    V* buf = reinterpret_cast<V*>(smraw);
+    static_assert(NB == 1, "ratios are of one bin a CTA");
+    float* buf = reinterpret_cast<float*>(smraw);
     if (run.x >= 0) {
 #pragma unroll
       for (int j = 0; j < R; j++)
-        if (j < run.z) buf[plane + j] = acc[j];
+        if (j < run.z) buf[plane + j] = acc[j].v[0];
     }
     __syncthreads();
     const size_t base = ((size_t)tl * g.nrad + ird) * g.PS;
-    // U rows of a thread at a time: their plane, then data loads are in flight together
-    constexpr int U = 4 / NB;
+    // U rows of a thread at a time: their planes, then their data loads, are in
+    // flight together (row by row, 62x62x63 voxels and 53 segments took 52 us, now 37)
+    constexpr int U = 4;
     for (int p0 = tid; p0 < g.PP; p0 += U * nt) {
       int pl[U];
 #pragma unroll
       for (int u = 0; u < U; u++) pl[u] = p0 + u * nt < g.PP ? a.rowplane[p0 + u * nt] : -1;
-      float2 db[U][NB];
-      float cal[U][NB];
+      float2 db[U];
+      float cal[U];
 #pragma unroll
       for (int u = 0; u < U; u++) {
         // pad rows: segment 0's repeat its first and last plane, the others are gaps
         const int p = p0 + u * nt, row = p == 0 ? 1 : (p == NZS + 1 ? NZS : p);
-#pragma unroll
-        for (int b = 0; b < NB; b++) {
-          const bool in = pl[u] >= 0 && (NB == 1 || ird + b < g.nrad);
-          const size_t o = base + (size_t)b * g.PS + row;
-          db[u][b] = in ? F.dbg[o] : make_float2(0.f, 0.f);
-          cal[u][b] = PAIRS && in ? F.cal[o] : -1000.f;
-        }
+        db[u] = pl[u] >= 0 ? F.dbg[base + row] : make_float2(0.f, 0.f);
+        cal[u] = PAIRS && pl[u] >= 0 ? F.cal[base + row] : -1000.f;
       }
 #pragma unroll
       for (int u = 0; u < U; u++) {
         const int p = p0 + u * nt;
         if (p >= g.PP) break;
-        V proj{};
-        if (pl[u] >= 0) proj = buf[pl[u]];
-#pragma unroll
-        for (int b = 0; b < NB; b++) {
-          if (NB > 1 && ird + b >= g.nrad) break;  // whole block
-          const size_t o = base + (size_t)b * g.PS;
-          const float s = __fadd_rn(proj.v[b], db[u][b].y);
-          const float corr = pl[u] >= 0 && s >= 0.01f ? __fdiv_rn(db[u][b].x, s) : -1000.f;
-          if constexpr (PAIRS) {
-            using P = typename PairT<STORE>::type;
-            static_cast<P*>(F.corr)[o + p] = pair_from<P>(make_float2(corr, cal[u][b]));
-          } else {
-            using T = typename ElemT<STORE>::type;
-            static_cast<T*>(F.corr)[o + p] = elem_from<T>(corr);
-          }
+        const float s = __fadd_rn(pl[u] >= 0 ? buf[pl[u]] : 0.f, db[u].y);
+        const float corr = pl[u] >= 0 && s >= 0.01f ? __fdiv_rn(db[u].x, s) : -1000.f;
+        if constexpr (PAIRS) {
+          using P = typename PairT<STORE>::type;
+          static_cast<P*>(F.corr)[base + p] = pair_from<P>(make_float2(corr, cal[u]));
+        } else {
+          using T = typename ElemT<STORE>::type;
+          static_cast<T*>(F.corr)[base + p] = elem_from<T>(corr);
         }
       }
     }
@@ -291,9 +281,9 @@ __global__ void __launch_bounds__(512, R == 9 && NB == 1 ? 2 : 1) fp_kernel(cons
 template <int R, int NB, bool RATIO, bool FULL, int STORE, bool PAIRS>
 static cudaError_t launch_fp_n(FpArgs a, const FpSchedule& s, int na, cudaStream_t st) {
   auto k = fp_kernel<R, NB, RATIO, FULL, STORE, PAIRS>;
-  if (NB > 1) a.lc = (s.lc + 1) / 2;  // 64 KB of columns at the default 32 steps, as many bytes as 64 steps of one bin
+  if (NB > 1) a.lc = (s.lc + 1) / 2;  // as many bytes as one bin's steps twice: 43 KB at the default 32 steps and 168 floats a column
   size_t smem = (size_t)a.lc * a.cw * sizeof(Bins<NB>) + (size_t)a.lc * NB * (sizeof(int4) + sizeof(float2));
-  if (RATIO) smem = std::max(smem, (size_t)a.g.P * sizeof(Bins<NB>));
+  if (RATIO) smem = std::max(smem, (size_t)a.g.P * sizeof(float));
   a.inv_nzq[0] = 1.f / (float)a.g.nzp;
   a.inv_nzq[1] = 2.f / (float)a.g.nzp;
   a.inv_nzq[2] = 4.f / (float)a.g.nzp;
@@ -304,28 +294,13 @@ static cudaError_t launch_fp_n(FpArgs a, const FpSchedule& s, int na, cudaStream
   return cudaGetLastError();
 }
 
-// Bins per CTA.  Four bins share the loads' addresses, a quarter of the warp's
-// conflicts and packed arithmetic, but make a quarter of the CTAs with twice
-// the registers: they pay where the grid is large.  One / four bins, us a
-// launch, by the threads of the one-bin grid: projections (layout kernel
-// included) 27 / 37 at 33 K (64x64x32, 16 angles), 81 / 73 at 221 K (96^3, 12
-// angles), 273 / 273 at 655 K (128x128x159, 53 segments, 10 angles: 320 CTAs
-// on 152 SMs; 247 / 191 where the next call's CTAs fill the last wave), 228 /
-// 201 at 0.5 M and 1641 / 1292 at 4 M (15 segments, 21 and 168 angles).  With the
-// ratio, whose data the fewer warps wait for, 76 / 82, 252 / 292, 220 / 223 and
-// 1576 / 1419; eight frames of 96^3 in one launch lose 6 % to it, so a group of
-// frames stays at one bin.
 template <int R, bool RATIO, bool FULL, int STORE, bool PAIRS>
 static cudaError_t launch_fp_t(const FpArgs& a, const FpSchedule& s, cudaStream_t st) {
   int na = 0;
   for (int f = 0; f < (a.nfr > 1 ? a.nfr : 1); f++) na = a.fr[f].na > na ? a.fr[f].na : na;
-  if constexpr (R == 9) {
-    const long long threads = (long long)a.g.nrad * na * (a.nfr > 1 ? a.nfr : 1) * s.nthreads;
-    const size_t smem4 = (size_t)std::max((s.lc + 1) / 2 * (a.cw + 6), a.g.P) * sizeof(Bins<4>);
-    if (RATIO ? a.nfr <= 1 && threads >= 2000000 : threads >= 150000)
-      if (smem4 <= 200 * 1024)
-        return launch_fp_n<R, 4, RATIO, FULL, STORE, PAIRS>(a, s, na, st);
-  }
+  if constexpr (R == 9 && !RATIO)
+    if (fp_bins(s, a.g.nseg, a.g.nrad, na * (a.nfr > 1 ? a.nfr : 1)) == 4)
+      return launch_fp_n<R, 4, RATIO, FULL, STORE, PAIRS>(a, s, na, st);
   return launch_fp_n<R, 1, RATIO, FULL, STORE, PAIRS>(a, s, na, st);
 }
 

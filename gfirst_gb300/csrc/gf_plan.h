@@ -79,6 +79,9 @@ struct FpSchedule {
 };
 bool make_fp_schedule(const Plan& p, int R, int lc, FpSchedule* out);
 int fp_default_R(const Plan& p);
+// Radial bins of a CTA (1 or 4) for projections without the ratio of `views`
+// (angle, frame) pairs.
+int fp_bins(const FpSchedule& s, int nseg, int nrad, int views);
 
 // The staged-row buffer of a plan (a context's Plan::pads holds it).
 BpPads bp_fast_pads(const Plan& p);

@@ -110,6 +110,10 @@ gf_status gf_bp_staged_rows(const gf_geometry* g, int32_t* pad_lo, int32_t* pad_
  * warp per column. */
 gf_status gf_bp_run(const gf_geometry* g, int32_t nsubsets, int32_t images, int32_t* slices);
 
+/* How gf_forward_project runs a subset with the default tile shapes (no device
+ * work): radial bins that one block projects together, 1 or 4. */
+gf_status gf_fp_run(const gf_geometry* g, int32_t nsubsets, int32_t subset, int32_t* bins);
+
 /* Device memory helpers for callers without a CUDA runtime of their own. */
 gf_status gf_device_alloc(gf_ctx* ctx, size_t bytes, void** d_ptr);
 gf_status gf_device_free(gf_ctx* ctx, void* d_ptr);
