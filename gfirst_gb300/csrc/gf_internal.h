@@ -127,9 +127,8 @@ struct gf_recon {
   float* proj_ref = nullptr;
   bool cyl_proj_ready = false;  // proj_ref holds the unit-cylinder projection (modes 1-3)
   float* proj_t = nullptr;  // triples projection, file layout (VLOR split weights)
-  int32_t* events = nullptr;
   unsigned long long* vlor_keys = nullptr;  // event ends sorted by (bin, event), 2*nev
-  float2* vlor_ends = nullptr;              // projection and weight of each event end's bin, 2*nev
+  float2* vlor_ends = nullptr;              // projection and weight of each event end's bin, 2*nev (a load sorts through it)
   int64_t nev = 0, ev_cap = 0;
   float* blankt = nullptr;
   float* datos_v = nullptr;

@@ -410,37 +410,39 @@ static gf_status load_impl(gf_recon* r, const float* h_image, const float* h_dsi
   if (mode == 3) {
     if (nevents != r->nev) r->gen++;  // the split's launch holds the count
     r->nev = nevents;
-    if (nevents > 0) {
-      if (nevents > r->ev_cap) {
-        // the smaller buffers go back to the pool before the larger ones are taken
-        r->release(r->events);
-        r->release(r->vlor_keys);
-        r->release(r->vlor_ends);
-        r->events = nullptr;
-        r->vlor_keys = nullptr;
-        r->vlor_ends = nullptr;
-        r->ev_cap = 0;
-        r->gen++;
-        if ((s = r->alloc_t((size_t)nevents * 2, &r->events)) != GF_OK) return done(s);
-        if ((s = r->alloc_t((size_t)nevents * 2, &r->vlor_keys)) != GF_OK) return done(s);
-        if ((s = r->alloc_t((size_t)nevents * 2, &r->vlor_ends)) != GF_OK) return done(s);
-        r->ev_cap = nevents;
-      }
-      if ((s = ck(cudaMemcpyAsync(r->events, h_events, (size_t)nevents * 2 * sizeof(int32_t), cudaMemcpyHostToDevice, st), "upload events")) != GF_OK) return done(s);
-      // the event ends in the order the VLOR split adds them (temporaries stream-ordered)
-      unsigned long long* keys_tmp = nullptr;
-      void* temp = nullptr;
-      const size_t tb = vlor_sort_temp_bytes(nevents);
-      cudaError_t e = cudaMallocAsync(&keys_tmp, (size_t)nevents * 2 * sizeof(unsigned long long), st);
-      if (e == cudaSuccess) e = cudaMallocAsync(&temp, tb ? tb : 16, st);
-      if (e == cudaSuccess) e = launch_vlor_sort(c->dg, r->events, nevents, keys_tmp, r->vlor_keys, temp, tb, st);
-      if (keys_tmp) cudaFreeAsync(keys_tmp, st);
-      if (temp) cudaFreeAsync(temp, st);
-      if ((s = ck(e, "sort VLOR events")) != GF_OK) return done(s);
+    if (nevents > r->ev_cap) {
+      // the smaller buffers go back to the pool before the larger ones are taken
+      r->release(r->vlor_keys);
+      r->release(r->vlor_ends);
+      r->vlor_keys = nullptr;
+      r->vlor_ends = nullptr;
+      r->ev_cap = 0;
+      r->gen++;
+      if ((s = r->alloc_t((size_t)nevents * 2, &r->vlor_keys)) != GF_OK) return done(s);
+      if ((s = r->alloc_t((size_t)nevents * 2, &r->vlor_ends)) != GF_OK) return done(s);
+      r->ev_cap = nevents;
     }
-    // counts in datos_v (scratch for now), then BLANKT (GFIRST.cu:229-247)
-    if ((s = ck(cudaMemsetAsync(r->datos_v, 0, pl.ndata * sizeof(float), st), "memset")) != GF_OK) return done(s);
-    if ((s = ck(launch_vlor_count(c->dg, r->events, nevents, r->datos_v, st), "vlor count")) != GF_OK) return done(s);
+    // The event ends in the order the VLOR split adds them, then the events'
+    // counts in datos_v (scratch for now); the events themselves are not needed
+    // after that (stream-ordered).
+    int32_t* ev = nullptr;
+    void* temp = nullptr;
+    cudaError_t e = cudaSuccess;
+    if (nevents > 0) {
+      static_assert(sizeof(*r->vlor_ends) == sizeof(*r->vlor_keys), "unsorted keys lie in vlor_ends");
+      const size_t tb = vlor_sort_temp_bytes(nevents);
+      e = cudaMallocAsync(&ev, (size_t)nevents * 2 * sizeof(int32_t), st);
+      if (e == cudaSuccess) e = cudaMallocAsync(&temp, tb ? tb : 16, st);
+      if (e == cudaSuccess) e = cudaMemcpyAsync(ev, h_events, (size_t)nevents * 2 * sizeof(int32_t), cudaMemcpyHostToDevice, st);
+      if (e == cudaSuccess)
+        e = launch_vlor_sort(c->dg, ev, nevents, reinterpret_cast<unsigned long long*>(r->vlor_ends), r->vlor_keys, temp, tb, st);
+    }
+    if (e == cudaSuccess) e = cudaMemsetAsync(r->datos_v, 0, pl.ndata * sizeof(float), st);
+    if (e == cudaSuccess) e = launch_vlor_count(c->dg, ev, nevents, r->datos_v, st);
+    if (ev) cudaFreeAsync(ev, st);
+    if (temp) cudaFreeAsync(temp, st);
+    if ((s = ck(e, "VLOR events")) != GF_OK) return done(s);
+    // BLANKT (GFIRST.cu:229-247)
     if ((s = ck(launch_blankt(c->dg, r->datos_v, s2, r->blankt, st), "blankt")) != GF_OK) return done(s);
   }
   // the staging is free again once the compute stream has passed the layout kernels

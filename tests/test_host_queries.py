@@ -30,3 +30,16 @@ def test_queries_do_not_size_the_staged_rows(query):
     for _ in range(20):
         query()
     assert time.perf_counter() - t < 2.0
+
+
+def test_an_event_costs_its_sorted_ends_and_their_values():
+    """2 ends a VLOR event: 8 bytes of key, 8 of projection and weight each."""
+    import ctypes
+
+    def total(events):
+        p, b = gf.recon_defaults(3), ctypes.c_int64()
+        g = gf.Geometry.small()
+        assert gf.lib().gf_recon_bytes(ctypes.byref(g.c()), 4, ctypes.byref(p), ctypes.c_int64(events), ctypes.byref(b)) == 0
+        return b.value
+
+    assert total(1000) - total(0) == 1000 * 32
