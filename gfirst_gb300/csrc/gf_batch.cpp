@@ -37,7 +37,7 @@ struct gf_batch {
   // per unit and member: its class (the first member with the same subset
   // count and an equal normalization mask), or -1
   std::vector<std::vector<int>> cls;
-  int* d_flag = nullptr;                // device flag of the mask comparison
+  int* d_flag = nullptr;                // device flags of the mask comparison, kMaxFrames
   cudaStream_t origin = nullptr;
   cudaEvent_t fork = nullptr;
   std::vector<cudaEvent_t> joins;  // one per frame (a unit uses its first frame's)
@@ -92,7 +92,8 @@ static void make_units(gf_batch* b) {
 // normalization masks (every subset, in that count's layout), compared on the
 // device after the frames' queued work (their loads) has finished.  Where the
 // back projector runs one warp per column such frames share it two by two;
-// to_run: only these are compared.
+// to_run: only these are compared.  The frames without a class are compared with
+// the first of them in one go, so the host waits once per class.
 static gf_status check_masks(const gf_batch* b, bool to_run, std::vector<std::vector<int>>* out) {
   std::vector<std::vector<int>> cls(b->units.size());
   for (size_t k = 0; k < b->units.size(); k++) {
@@ -101,32 +102,30 @@ static gf_status check_masks(const gf_batch* b, bool to_run, std::vector<std::ve
     if (b->fused != 1 || u.size() < 2) continue;
     if (b->frames[u[0]]->ctx->bp_form != GF_BP_PER_VIEW) continue;
     if (to_run && !b->frames[u[0]]->cal) continue;  // column tiles take each frame on its own
-    for (size_t j = 0; j < u.size(); j++) {
-      const gf_recon* r = b->frames[u[j]];
-      cls[k][j] = (int)j;  // a class of its own unless an earlier leader matches
-      for (size_t i = 0; i < j; i++) {
-        if (cls[k][i] != (int)i) continue;  // not a class leader
-        const gf_recon* l = b->frames[u[i]];
-        if (l->ctx->plan.nsub != r->ctx->plan.nsub) continue;
-        bool same = false;
-        {
-          GF_CK(cudaStreamSynchronize(l->ctx->stream));
-          GF_CK(cudaStreamSynchronize(r->ctx->stream));
-          // the same geometry and subset count: the same form on both sides
-          const float* ml = l->cal ? l->cal : reinterpret_cast<const float*>(l->mask);
-          const float* mr = r->cal ? r->cal : reinterpret_cast<const float*>(r->mask);
-          const size_t n = l->cal ? (size_t)l->ctx->plan.all_elems() : l->mask_words();
-          GF_CK(launch_differs(ml, mr, n, b->d_flag, b->origin));
-          int flag = 1;
-          GF_CK(cudaMemcpyAsync(&flag, b->d_flag, sizeof(int), cudaMemcpyDeviceToHost, b->origin));
-          GF_CK(cudaStreamSynchronize(b->origin));
-          same = flag == 0;
-        }
-        if (same) {
-          cls[k][j] = (int)i;
-          break;
-        }
+    for (int i : u) {
+      GF_CK(cudaEventRecord(b->joins[i], b->frames[i]->ctx->stream));
+      GF_CK(cudaStreamWaitEvent(b->origin, b->joins[i], 0));
+    }
+    for (size_t i = 0; i < u.size(); i++) {
+      if (cls[k][i] >= 0) continue;
+      cls[k][i] = (int)i;
+      const gf_recon* l = b->frames[u[i]];
+      // the same geometry and subset count: the same form on both sides
+      auto bits = [](const gf_recon* r) { return r->cal ? r->cal : reinterpret_cast<const float*>(r->mask); };
+      const size_t n = l->cal ? (size_t)l->ctx->plan.all_elems() : l->mask_words();
+      std::vector<size_t> with;
+      for (size_t j = i + 1; j < u.size(); j++) {
+        const gf_recon* r = b->frames[u[j]];
+        if (cls[k][j] >= 0 || l->ctx->plan.nsub != r->ctx->plan.nsub) continue;
+        GF_CK(launch_differs(bits(l), bits(r), n, b->d_flag + with.size(), b->origin));
+        with.push_back(j);
       }
+      if (with.empty()) continue;
+      int differs[kMaxFrames];
+      GF_CK(cudaMemcpyAsync(differs, b->d_flag, with.size() * sizeof(int), cudaMemcpyDeviceToHost, b->origin));
+      GF_CK(cudaStreamSynchronize(b->origin));
+      for (size_t q = 0; q < with.size(); q++)
+        if (!differs[q]) cls[k][with[q]] = (int)i;
     }
   }
   *out = std::move(cls);
@@ -180,7 +179,7 @@ gf_status gf_batch_create(int32_t n, gf_recon* const* frames, gf_batch** out) {
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
   b->joins.assign(n, nullptr);
   for (int i = 0; i < n && e == cudaSuccess; i++) e = cudaEventCreateWithFlags(&b->joins[i], cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaMalloc(&b->d_flag, sizeof(int));
+  if (e == cudaSuccess) e = cudaMalloc(&b->d_flag, kMaxFrames * sizeof(int));
   if (e != cudaSuccess) {
     gf_batch_destroy(b);
     return cuda_error(e, "batch set-up");
