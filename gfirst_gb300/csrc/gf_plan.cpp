@@ -200,9 +200,13 @@ static BpTile tile_shape(const Plan& p, int warps, int elem_bytes, int zr) {
   const double diag = std::hypot((double)(cx - 1), (double)(cy - 1));
   double fzmax = 0;
   for (const Seg& s : p.seg) fzmax = std::max(fzmax, (double)std::fabs(s.fz));
-  // floor(x + d) - floor(x) <= floor(d) + 1; the 1e-3 covers float rounding
-  const double nb = std::floor(diag * p.fx_bp + 1e-3) + 3;
-  const double spread = std::floor(diag * fzmax + 1e-3) + 1;
+  // floor(x + d) - floor(x) <= floor(d) + 1; the 2e-3 covers float rounding: with
+  // 1024 columns, 4096 bins and slots of at most 10 KB (fx up to 3.6), each of two
+  // corners' bins is off by at most 0.5 ulp in two products and their sum (6e-5 fx),
+  // in the scaled sum (6e-5) and in the two additions after it (1.2e-4 each): 1.03e-3
+  // together; a row (fz up to 12 before the image's slices bound the rows) by less
+  const double nb = std::floor(diag * p.fx_bp + 2e-3) + 3;
+  const double spread = std::floor(diag * fzmax + 2e-3) + 1;
   const int ve = 16 / elem_bytes;
   t.nb = (int)std::min((double)p.g.nrad, nb);
   t.rows = (int)std::min((double)(p.g.nzs + 2), (double)t.zr + spread + 2);
