@@ -192,7 +192,8 @@ __device__ __forceinline__ void segment_views(float2 (&acc)[Q], const float (&fi
   // prefetch their first three chunks and load the others while staging: that
   // fits 64 registers too, and the eighth resident block per SM hides more
   // than the exposed loads cost (1.294 ms; all chunks prefetched at 72
-  // registers, seven blocks: 1.336 ms; at 80 registers, six blocks: 1.343 ms).
+  // registers, seven blocks: 1.336 ms; at 80 registers, six blocks: 1.343 ms; at
+  // 128x128x159 voxels, which run tiles now: not measured at the sizes left here).
   {
     constexpr int PF = (sizeof(Pair) == 8 && NCH > bp_pf32<FAST>) ? bp_pf32<FAST> : NCH;
     Pair c0[PF], c1[PF];
@@ -519,7 +520,9 @@ __global__ void __launch_bounds__(256) __maxnreg__(bp_pair_regs<STORE>) bp_pair_
 // to 160 slices both pair types are capped at 64 registers (eight 4-warp
 // blocks per SM, no spill; FP32 with the shallower prefetch above) -- 1.296
 // and 1.245 ms against 1.343 and 1.264 ms under the launch bounds of
-// bp_kernel_deep (six and eight blocks).  The cap is a constant that depends
+// bp_kernel_deep (six and eight blocks), at 128x128x159 voxels, which run tiles
+// now; columns of one or two chunks, the most of what is left here, need fewer
+// registers and were not measured apart.  The cap is a constant that depends
 // on the template argument, so it stands beside the 256-thread bound (both
 // reach the compiled kernel); the cap alone, or a (128, 8) launch bound,
 // schedules worse: 1.340 and 1.266 ms.  Deeper columns keep the launch

@@ -352,7 +352,8 @@ __global__ void __launch_bounds__(256) bp_tile_kernel(const BpArgs a) {
     const bool tiny = ok != range && (fminf(wa, al) * fminf(wl, be) <= kTinyWeight || edge);
     // The lanes' ranges differ by little: most runs at an edge have stretches
     // that no lane needs.
-    constexpr int ZG = ZR % 5 == 0 ? 5 : 4;
+    constexpr int ZG = 4;
+    static_assert(ZR % ZG == 0, "whole stretches");
     const unsigned some = __reduce_or_sync(kAll, ok);
     auto masked = [&](auto one) {
 #pragma unroll

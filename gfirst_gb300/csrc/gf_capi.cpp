@@ -295,7 +295,7 @@ gf_status gf_create(const gf_geometry* g, int32_t nsubsets, int32_t device, gf_c
   std::vector<int4> runs(c->fps.runs.size());
   for (size_t i = 0; i < runs.size(); i++) {
     const Run& r = c->fps.runs[i];
-    runs[i] = make_int4(r.seg, r.p0, r.n, r.pad);
+    runs[i] = make_int4(r.seg, r.p0, r.n, 0);
   }
   gf_status st;
   if ((st = c->alloc_t(segs.size(), &c->d_seg)) != GF_OK) return fail(st);

@@ -71,9 +71,8 @@ __device__ __forceinline__ void add_sample(Bins<NB>& acc, const Bins<NB>& a, con
 template <int NB>
 __device__ __forceinline__ Bins<NB> ldg_bins(const float* p) {
   Bins<NB> r;
-  if constexpr (NB == 1) {
-    r.v[0] = __ldg(p);
-  } else if constexpr (NB == 2) {
+  static_assert(NB == 2 || NB == 4, "a vector load");
+  if constexpr (NB == 2) {
     const float2 v = __ldg(reinterpret_cast<const float2*>(p));
     r.v[0] = v.x;
     r.v[1] = v.y;
@@ -154,7 +153,7 @@ __global__ void __launch_bounds__(512, R == 9 && NB == 1 ? 2 : 1) fp_kernel(cons
     // ZV slices a thread: one 4 ZV-byte load per corner column
     const int nzq = NZP / ZV;
     for (int idx = tid; idx < nl * nzq; idx += nt) {
-      const int l = (int)(((float)idx + 0.5f) * a.inv_nzq[ZV >> 1]), z = (idx - l * nzq) * ZV;
+      const int l = (int)(((float)idx + 0.5f) * a.inv_nzq[ZV == 4]), z = (idx - l * nzq) * ZV;
       V c[ZV];
 #pragma unroll
       for (int b = 0; b < NB; b++) {
@@ -284,9 +283,8 @@ static cudaError_t launch_fp_n(FpArgs a, const FpSchedule& s, int na, cudaStream
   if (NB > 1) a.lc = (s.lc + 1) / 2;  // as many bytes as one bin's steps twice: 43 KB at the default 32 steps and 168 floats a column
   size_t smem = (size_t)a.lc * a.cw * sizeof(Bins<NB>) + (size_t)a.lc * NB * (sizeof(int4) + sizeof(float2));
   if (RATIO) smem = std::max(smem, (size_t)a.g.P * sizeof(float));
-  a.inv_nzq[0] = 1.f / (float)a.g.nzp;
-  a.inv_nzq[1] = 2.f / (float)a.g.nzp;
-  a.inv_nzq[2] = 4.f / (float)a.g.nzp;
+  a.inv_nzq[0] = 2.f / (float)a.g.nzp;
+  a.inv_nzq[1] = 4.f / (float)a.g.nzp;
   cudaError_t e = allow_max_smem(k);
   if (e != cudaSuccess) return e;
   dim3 grid((a.g.nrad + NB - 1) / NB, na, a.nfr > 1 ? a.nfr : 1);

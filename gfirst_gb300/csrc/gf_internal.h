@@ -66,7 +66,7 @@ struct gf_ctx {
   // Bumped whenever a launch parameter that a captured graph holds changes
   // (the projectors' tile shapes, gf_tune); gf_batch recaptures on a change.
   int64_t gen = 0;
-  int bp_warps = 4;      // back-projector warps (slice runs of one column tile) per block
+  int bp_warps = 4;      // back-projector warps per block: neighbouring column tiles of one run, or image columns
   // back projector's axial interpolation for doubles images and the operator
   // entry point (gf_set_bp_form); triples images always use GF_BP_PER_VOXEL
   int bp_form = GF_BP_PER_VIEW;

@@ -43,10 +43,10 @@ struct FpFrame {
 };
 struct FpArgs {
   DevGeom g;               // g.nsub unused: each frame names its own
-  const int4* runs;        // FpSchedule::runs as (seg, p0, n, pad)
+  const int4* runs;        // FpSchedule::runs as (seg, p0, n, -)
   int nruns, padl, cw, lc;
   const int* rowplane;     // per padded row: its plane (segment 0's pad rows: the edge plane), -1 a gap; with corr
-  float inv_nzq[3];        // set by launch_fp: 1, 2 and 4 slices over the column's
+  float inv_nzq[2];        // set by launch_fp: 2 and 4 slices over the column's
   int storage;             // ratio element type: 0 float, 1 __half, 2 __nv_bfloat16
   int nfr;                 // frames in this launch (grid z); 0 is taken as 1
   FpFrame fr[kMaxFrames];

@@ -85,7 +85,7 @@ extern "C" gf_status gf_forward_project_noalloc(const gf_geometry* gg, int32_t n
   std::vector<float2> trig(geo.nang);
   for (int t = 0; t < geo.nang; t++) trig[t] = make_float2(plan.sinv[t], plan.cosv[t]);
   std::vector<int4> runs(fps.runs.size());
-  for (size_t i = 0; i < runs.size(); i++) runs[i] = make_int4(fps.runs[i].seg, fps.runs[i].p0, fps.runs[i].n, fps.runs[i].pad);
+  for (size_t i = 0; i < runs.size(); i++) runs[i] = make_int4(fps.runs[i].seg, fps.runs[i].p0, fps.runs[i].n, 0);
   // pageable sources: each copy has read its source when the call returns
   GF_CK(cudaMemcpyAsync(dseg, segs.data(), segs.size() * sizeof(DevSeg), cudaMemcpyHostToDevice, st));
   GF_CK(cudaMemcpyAsync(dtrig, trig.data(), trig.size() * sizeof(float2), cudaMemcpyHostToDevice, st));

@@ -97,10 +97,7 @@ bool make_fp_schedule(const Plan& p, int R, int lc, FpSchedule* out) {
     const Seg& sg = p.seg[s];
     int end = p.g.nzs - sg.zmin;
     for (int p0 = sg.zmin; p0 < end; p0 += R) {
-      Run r{s, p0, std::min(R, end - p0), 0};
-      if (p0 == sg.zmin) r.pad |= 1;
-      if (p0 + r.n == end) r.pad |= 2;
-      f.runs.push_back(r);
+      f.runs.push_back(Run{s, p0, std::min(R, end - p0)});
       for (int lam : {p.lam0, p.lam1}) {
         float t = (float)lam * sg.dz;
         int m = (int)floorf(t);
@@ -205,18 +202,18 @@ static BpTile tile_shape(const Plan& p, int warps, int elem_bytes, int zr) {
   // corners' bins is off by at most 0.5 ulp in two products and their sum (6e-5 fx),
   // in the scaled sum (6e-5) and in the two additions after it (1.2e-4 each): 1.03e-3
   // together; a row (fz up to 12 before the image's slices bound the rows) by less
-  const double nb = std::floor(diag * p.fx_bp + 2e-3) + 3;
+  const double nbins = std::floor(diag * p.fx_bp + 2e-3) + 3;
   const double spread = std::floor(diag * fzmax + 2e-3) + 1;
   const int ve = 16 / elem_bytes;
-  t.nb = (int)std::min((double)p.g.nrad, nb);
-  t.rows = (int)std::min((double)(p.g.nzs + 2), (double)t.zr + spread + 2);
+  const int nb = (int)std::min((double)p.g.nrad, nbins);  // radial bins and rows of a view at most
+  const int rows = (int)std::min((double)(p.g.nzs + 2), (double)t.zr + spread + 2);
   // bins 4 words apart modulo 8 (16-byte copies, few bank conflicts)
-  int words = ((t.rows + 2 * (ve - 1)) * elem_bytes + 3) / 4;
+  int words = ((rows + 2 * (ve - 1)) * elem_bytes + 3) / 4;
   words += (12 - words % 8) % 8;
   t.rs = words * 4 / elem_bytes;
-  t.mw = (t.rows + 62) / 32 + 2;
-  t.rows_at = (48 + 4 * t.nb * t.mw + 15) / 16 * 16;
-  t.slot_bytes = (t.rows_at + (bp_pad_front(t.zr, elem_bytes) + t.nb * t.rs + t.zr + 2) * elem_bytes + 15) / 16 * 16;
+  t.mw = (rows + 62) / 32 + 2;
+  t.rows_at = (48 + 4 * nb * t.mw + 15) / 16 * 16;
+  t.slot_bytes = (t.rows_at + (bp_pad_front(t.zr, elem_bytes) + nb * t.rs + t.zr + 2) * elem_bytes + 15) / 16 * 16;
   return t;
 }
 

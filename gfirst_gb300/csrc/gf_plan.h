@@ -34,7 +34,7 @@ struct Seg {
 
 // One forward-projector thread's run of consecutive planes in one segment.
 struct Run {
-  int seg, p0, n, pad;  // pad: bit0 = writes the row before, bit1 = after
+  int seg, p0, n;
 };
 
 // Staged-row buffer of the back projector's per-view form: each warp stages a
@@ -88,8 +88,8 @@ BpPads bp_fast_pads(const Plan& p);
 
 // Shape of the back projector's work.  Column tiles (gf_bp_tile.cu): a warp owns
 // kTileX x kTileY columns and a run of zr slices (kTileRun, or kShortRun where
-// that makes few CTAs), a CTA `warps` such tiles (two in y) and one run.  zr = 0: one warp per column (gf_bp.cu), `warps`
-// a block.
+// that makes few CTAs), a CTA `warps` such tiles (two in y) and one run.  zr = 0:
+// one warp per column (gf_bp.cu), `warps` a block.
 constexpr int kTileX = 4, kTileY = 8, kTileRun = 12, kShortRun = 8;
 // Elements before a staged view's first row: a lane's run may start that far
 // before the segment's rows.
@@ -98,7 +98,6 @@ constexpr int bp_pad_front(int zr, int elem_bytes) {
 }
 struct BpTile {
   int zr = 0, warps = 0;
-  int nb = 0, rows = 0;     // radial bins and rows of one view at most
   int rs = 0, mw = 0;       // row stride of a bin (elements), mask words of a bin
   int rows_at = 0, slot_bytes = 0;
   BpPads pads;              // one warp per column

@@ -2,7 +2,7 @@
 //
 // Forward projector: R (planes per thread run; odd, so a warp's shared loads
 // fall in distinct banks) and the number of ray steps staged per shared-memory
-// chunk.  Back projector: warps (image columns) per block.  Each candidate
+// chunk.  Back projector: warps per block (a column tile or an image column each).  Each candidate
 // runs once to warm up and three times under CUDA events on subset 0 of the
 // context's geometry with a unit-cylinder image; the fastest is kept.
 #include <vector>
@@ -27,7 +27,7 @@ struct Timer {
 
 gf_status upload_runs(gf_ctx* c, const FpSchedule& f) {
   std::vector<int4> runs(f.runs.size());
-  for (size_t i = 0; i < runs.size(); i++) runs[i] = make_int4(f.runs[i].seg, f.runs[i].p0, f.runs[i].n, f.runs[i].pad);
+  for (size_t i = 0; i < runs.size(); i++) runs[i] = make_int4(f.runs[i].seg, f.runs[i].p0, f.runs[i].n, 0);
   GF_CK(cudaMemcpyAsync(c->d_runs, runs.data(), runs.size() * sizeof(int4), cudaMemcpyHostToDevice, c->stream));
   GF_CK(cudaStreamSynchronize(c->stream));
   return GF_OK;
