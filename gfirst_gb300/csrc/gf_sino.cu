@@ -198,6 +198,7 @@ __global__ void __launch_bounds__(256) ratio_from_file_kernel(const DevGeom g, c
   const int r0 = blockIdx.x * 32, p0 = blockIdx.y * 32, tl = blockIdx.z;
   const int theta = subset_angle(g, subset, tl);
   const int tx = threadIdx.x, ty = threadIdx.y;
+  bool other = false;
 #pragma unroll
   for (int k = 0; k < 4; k++) {
     const int p = p0 + ty + 8 * k, r = r0 + tx;
@@ -210,9 +211,16 @@ __global__ void __launch_bounds__(256) ratio_from_file_kernel(const DevGeom g, c
     }
     tc[ty + 8 * k][tx] = c;
     tm[ty + 8 * k][tx] = m;
+    other |= !(m == 1.f || m == -1000.f);
   }
-  __syncthreads();
-  bool other = false;
+  if (PAIRS) {
+    __syncthreads();
+  } else if (__syncthreads_or(other)) {
+    // the tiles will not run: one store a block and no bits (gf_back_project of 21
+    // angles x 1293 planes of other values all over: 724 us; 745 with both)
+    if (tx == 0 && ty == 0) *general = 1;
+    return;
+  }
 #pragma unroll
   for (int k = 0; k < 4; k++) {
     const int r = r0 + ty + 8 * k;
@@ -223,12 +231,10 @@ __global__ void __launch_bounds__(256) ratio_from_file_kernel(const DevGeom g, c
         static_cast<float2*>(out)[at * g.PS + p0 + tx] = make_float2(c, m);
       } else {
         static_cast<float*>(out)[at * g.PS + p0 + tx] = c;
-        other |= !(m == 1.f || m == -1000.f);
         put_mask_word(g, rowmap, at, p0, tx, m == 1.f, mask, dirty);
       }
     }
   }
-  if (!PAIRS && __any_sync(0xffffffffu, other) && tx == 0) *general = 1;
 }
 
 cudaError_t launch_ratio_from_file(const DevGeom& g, const int2* rowmap, int subset, int na, const float* corr,
