@@ -30,6 +30,13 @@ __device__ __forceinline__ bool resolve_row(const DevGeom& g, int2 m, int* seg, 
   return true;
 }
 
+// The sinogram plane that padded row p holds or repeats, -1 for a gap: plane k of
+// segment s is row k + 2 s + 1, so the segments' table is not needed.
+__device__ __forceinline__ int row_plane(int p, int2 m, int nzs) {
+  if (m.x < 0 || (m.y < 0 && m.x != 0)) return -1;
+  return m.y >= 0 ? p - 2 * m.x - 1 : (m.y == -1 ? 0 : nzs - 1);
+}
+
 // Rank of angle theta in the all-subset layout: subsets are stored in order,
 // subset s = theta % nsub holding angles s, s + nsub, ...; the first
 // nang % nsub subsets hold one angle more than the others.
@@ -198,20 +205,27 @@ __global__ void __launch_bounds__(256) ratio_from_file_kernel(const DevGeom g, c
   const int r0 = blockIdx.x * 32, p0 = blockIdx.y * 32, tl = blockIdx.z;
   const int theta = subset_angle(g, subset, tl);
   const int tx = threadIdx.x, ty = threadIdx.y;
+  const int r = min(r0 + tx, g.nrad - 1);
+  // the rows' planes first, then their data: two waits instead of two a row
+  int pl[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const int p = p0 + ty + 8 * k;
+    pl[k] = row_plane(p, rowmap[p], g.nzs);
+  }
+  float c[4], m[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const size_t lor = (size_t)pl[k] * ((size_t)g.nrad * g.nang) + (size_t)theta * g.nrad + r;
+    c[k] = pl[k] >= 0 ? corr[lor] : -1000.f;
+    m[k] = pl[k] >= 0 ? calib[lor] : -1000.f;
+  }
   bool other = false;
 #pragma unroll
   for (int k = 0; k < 4; k++) {
-    const int p = p0 + ty + 8 * k, r = r0 + tx;
-    float c = -1000.f, m = -1000.f;
-    int seg, plane;
-    if (p < g.PS && r < g.nrad && resolve_row(g, rowmap[p], &seg, &plane)) {
-      const size_t lor = file_lor(g, seg, plane, theta, r);
-      c = corr[lor];
-      m = calib[lor];
-    }
-    tc[ty + 8 * k][tx] = c;
-    tm[ty + 8 * k][tx] = m;
-    other |= !(m == 1.f || m == -1000.f);
+    tc[ty + 8 * k][tx] = c[k];
+    tm[ty + 8 * k][tx] = m[k];
+    other |= !(m[k] == 1.f || m[k] == -1000.f);
   }
   if (PAIRS) {
     __syncthreads();
