@@ -98,7 +98,7 @@ FpArgs gf_ctx::fp_args(int subset, const float* img_zfast) const {
   a.padl = fps.padl;
   a.cw = fps.cw;
   a.lc = fps.lc;
-  a.rowplane = d_rowplane;
+  a.rowmap = d_rowmap;
   return a;
 }
 
@@ -287,11 +287,6 @@ gf_status gf_create(const gf_geometry* g, int32_t nsubsets, int32_t device, gf_c
     for (int k = 0; k < sg.nplanes; k++) rowmap[sg.blk + 1 + k] = make_int2(s, sg.zmin + k);
     rowmap[sg.blk + sg.nplanes + 1] = make_int2(s, -2);
   }
-  std::vector<int> rowplane(p.PS, -1);
-  for (int s = 0; s < p.g.nseg; s++)
-    for (int k = 0; k < p.seg[s].nplanes; k++) rowplane[p.seg[s].blk + 1 + k] = p.seg[s].acc + k;
-  rowplane[0] = 0;
-  rowplane[p.g.nzs + 1] = p.g.nzs - 1;
   std::vector<int4> runs(c->fps.runs.size());
   for (size_t i = 0; i < runs.size(); i++) {
     const Run& r = c->fps.runs[i];
@@ -301,12 +296,10 @@ gf_status gf_create(const gf_geometry* g, int32_t nsubsets, int32_t device, gf_c
   if ((st = c->alloc_t(segs.size(), &c->d_seg)) != GF_OK) return fail(st);
   if ((st = c->alloc_t(trig.size(), &c->d_trig)) != GF_OK) return fail(st);
   if ((st = c->alloc_t(rowmap.size(), &c->d_rowmap)) != GF_OK) return fail(st);
-  if ((st = c->alloc_t(rowplane.size(), &c->d_rowplane)) != GF_OK) return fail(st);
   if ((st = c->alloc_t(512, &c->d_runs)) != GF_OK) return fail(st);  // room for any schedule (<= 512 threads)
   cudaMemcpyAsync(c->d_seg, segs.data(), segs.size() * sizeof(DevSeg), cudaMemcpyHostToDevice, c->stream);
   cudaMemcpyAsync(c->d_trig, trig.data(), trig.size() * sizeof(float2), cudaMemcpyHostToDevice, c->stream);
   cudaMemcpyAsync(c->d_rowmap, rowmap.data(), rowmap.size() * sizeof(int2), cudaMemcpyHostToDevice, c->stream);
-  cudaMemcpyAsync(c->d_rowplane, rowplane.data(), rowplane.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream);
   cudaMemcpyAsync(c->d_runs, runs.data(), runs.size() * sizeof(int4), cudaMemcpyHostToDevice, c->stream);
   if ((e = cudaStreamSynchronize(c->stream)) != cudaSuccess) return fail(cuda_error(e, "table upload"));
   DevGeom& d = c->dg;

@@ -45,6 +45,12 @@ template <> __device__ __forceinline__ __nv_bfloat16 elem_from<__nv_bfloat16>(fl
 
 __device__ __forceinline__ float lerp_rn(float a, float b, float w) { return __fmaf_rn(w, __fsub_rn(b, a), a); }
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return min(max(v, lo), hi); }
+// The sinogram plane that padded row p holds or repeats, -1 for a gap: plane k of
+// segment s is row k + 2 s + 1, so the segments' table is not needed.
+__device__ __forceinline__ int row_plane(int p, int2 m, int nzs) {
+  if (m.x < 0 || (m.y < 0 && m.x != 0)) return -1;
+  return m.y >= 0 ? p - 2 * m.x - 1 : (m.y == -1 ? 0 : nzs - 1);
+}
 // The update ratio of divVxVGPU (GFIRST_GPU_Kernels.cu:173-182): NUMER/DENOM,
 // 1 where DENOM < 0.001.
 __device__ __forceinline__ float update_ratio(float n, float d) { return d < 0.001f ? 1.0f : __fdiv_rn(n, d); }

@@ -249,7 +249,10 @@ __global__ void __launch_bounds__(512, R == 9 && NB == 1 ? 2 : 1) fp_kernel(cons
     for (int p0 = tid; p0 < g.PP; p0 += U * nt) {
       int pl[U];
 #pragma unroll
-      for (int u = 0; u < U; u++) pl[u] = p0 + u * nt < g.PP ? a.rowplane[p0 + u * nt] : -1;
+      for (int u = 0; u < U; u++) {
+        const int p = p0 + u * nt;
+        pl[u] = p < g.PP ? row_plane(p, a.rowmap[p], NZS) : -1;
+      }
       float2 db[U];
       float cal[U];
 #pragma unroll

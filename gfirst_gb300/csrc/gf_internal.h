@@ -59,7 +59,6 @@ struct gf_ctx {
   gf::DevSeg* d_seg = nullptr;
   float2* d_trig = nullptr;
   int2* d_rowmap = nullptr;
-  int* d_rowplane = nullptr;  // per padded row: FpArgs::rowplane
   int4* d_runs = nullptr;
   // scratch of the operator entry points, allocated on first use
   int64_t launches = 0;  // kernels launched by this context

@@ -45,7 +45,7 @@ struct FpArgs {
   DevGeom g;               // g.nsub unused: each frame names its own
   const int4* runs;        // FpSchedule::runs as (seg, p0, n, -)
   int nruns, padl, cw, lc;
-  const int* rowplane;     // per padded row: its plane (segment 0's pad rows: the edge plane), -1 a gap; with corr
+  const int2* rowmap;      // per padded row: (segment, plane or pad); with corr
   float inv_nzq[2];        // set by launch_fp: 2 and 4 slices over the column's
   int storage;             // ratio element type: 0 float, 1 __half, 2 __nv_bfloat16
   int nfr;                 // frames in this launch (grid z); 0 is taken as 1

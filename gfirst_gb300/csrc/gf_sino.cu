@@ -30,13 +30,6 @@ __device__ __forceinline__ bool resolve_row(const DevGeom& g, int2 m, int* seg, 
   return true;
 }
 
-// The sinogram plane that padded row p holds or repeats, -1 for a gap: plane k of
-// segment s is row k + 2 s + 1, so the segments' table is not needed.
-__device__ __forceinline__ int row_plane(int p, int2 m, int nzs) {
-  if (m.x < 0 || (m.y < 0 && m.x != 0)) return -1;
-  return m.y >= 0 ? p - 2 * m.x - 1 : (m.y == -1 ? 0 : nzs - 1);
-}
-
 // Rank of angle theta in the all-subset layout: subsets are stored in order,
 // subset s = theta % nsub holding angles s, s + nsub, ...; the first
 // nang % nsub subsets hold one angle more than the others.
