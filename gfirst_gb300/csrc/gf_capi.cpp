@@ -565,19 +565,19 @@ gf_status gf_vlor_split(gf_ctx* c, const int32_t* d_ev, int64_t n, const float* 
   // added in event order: the reference's sums, no atomics
   cudaStream_t st = c->stream;
   unsigned long long *keys_tmp = nullptr, *keys = nullptr;
-  float2* ends = nullptr;
+  float2* vals = nullptr;
   void* temp = nullptr;
   const size_t tb = vlor_sort_temp_bytes(n);
   cudaError_t e = cudaMallocAsync(&keys_tmp, (size_t)n * 2 * sizeof(unsigned long long), st);
   if (e == cudaSuccess) e = cudaMallocAsync(&keys, (size_t)n * 2 * sizeof(unsigned long long), st);
-  if (e == cudaSuccess) e = cudaMallocAsync(&ends, (size_t)n * 2 * sizeof(float2), st);
+  if (e == cudaSuccess) e = cudaMallocAsync(&vals, (size_t)n * (vlor_by_event(c->dg) ? 1 : 2) * sizeof(float2), st);
   if (e == cudaSuccess) e = cudaMallocAsync(&temp, tb ? tb : 16, st);
   if (e == cudaSuccess) e = launch_vlor_sort(c->dg, d_ev, n, keys_tmp, keys, temp, tb, st);
-  if (e == cudaSuccess) e = launch_vlor_split_sorted(c->dg, keys, n, d_proj, d_blankt, ends, d_out, st);
+  if (e == cudaSuccess) e = launch_vlor_split_sorted(c->dg, keys, n, d_ev, d_proj, d_blankt, vals, d_out, st);
   if (e == cudaSuccess) c->launches += 4;
   if (keys_tmp) cudaFreeAsync(keys_tmp, st);
   if (keys) cudaFreeAsync(keys, st);
-  if (ends) cudaFreeAsync(ends, st);
+  if (vals) cudaFreeAsync(vals, st);
   if (temp) cudaFreeAsync(temp, st);
   if (e != cudaSuccess) {
     cudaGetLastError();

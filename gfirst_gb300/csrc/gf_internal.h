@@ -127,7 +127,9 @@ struct gf_recon {
   bool cyl_proj_ready = false;  // proj_ref holds the unit-cylinder projection (modes 1-3)
   float* proj_t = nullptr;  // triples projection, file layout (VLOR split weights)
   unsigned long long* vlor_keys = nullptr;  // event ends sorted by (bin, event), 2*nev
-  float2* vlor_ends = nullptr;              // projection and weight of each event end's bin, 2*nev (a load sorts through it)
+  // 16 bytes an event, through which a load sorts: projection and weight of each
+  // end's bin, or (vlor_by_event) the events and, from nev on, their shares
+  float2* vlor_vals = nullptr;
   int64_t nev = 0, ev_cap = 0;
   float* blankt = nullptr;
   float* datos_v = nullptr;

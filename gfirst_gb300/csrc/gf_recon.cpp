@@ -105,7 +105,8 @@ gf_status gf_recon::subiteration(int t, int s) {
     stage_end();
     stage_begin(GF_STAGE_VLOR);
     GF_CK(cudaMemsetAsync(datos_v, 0, (size_t)pl.ndata * sizeof(float), st));
-    GF_LAUNCH(c, launch_vlor_split_sorted(c->dg, vlor_keys, nev, proj_t, blankt, vlor_ends, datos_v, st));
+    GF_LAUNCH(c, launch_vlor_split_sorted(c->dg, vlor_keys, nev, reinterpret_cast<const int32_t*>(vlor_vals), proj_t, blankt,
+                                          vlor_vals + (vlor_by_event(c->dg) ? nev : 0), datos_v, st));
     GF_LAUNCH(c, launch_ratio_gather(c->dg, c->d_rowmap, s, na, proj_t, datos_v, dbg[1] + off, cal_of(s), corr, p.storage, st));
     stage_end();
   } else {
@@ -413,32 +414,34 @@ static gf_status load_impl(gf_recon* r, const float* h_image, const float* h_dsi
     if (nevents > r->ev_cap) {
       // the smaller buffers go back to the pool before the larger ones are taken
       r->release(r->vlor_keys);
-      r->release(r->vlor_ends);
+      r->release(r->vlor_vals);
       r->vlor_keys = nullptr;
-      r->vlor_ends = nullptr;
+      r->vlor_vals = nullptr;
       r->ev_cap = 0;
       r->gen++;
       if ((s = r->alloc_t((size_t)nevents * 2, &r->vlor_keys)) != GF_OK) return done(s);
-      if ((s = r->alloc_t((size_t)nevents * 2, &r->vlor_ends)) != GF_OK) return done(s);
+      if ((s = r->alloc_t((size_t)nevents * 2, &r->vlor_vals)) != GF_OK) return done(s);
       r->ev_cap = nevents;
     }
     // The event ends in the order the VLOR split adds them, then the events'
-    // counts in datos_v (scratch for now); the events themselves are not needed
-    // after that (stream-ordered).
+    // counts in datos_v (scratch for now); the events themselves are kept only
+    // where the split walks them (stream-ordered).
     int32_t* ev = nullptr;
     void* temp = nullptr;
     cudaError_t e = cudaSuccess;
     if (nevents > 0) {
-      static_assert(sizeof(*r->vlor_ends) == sizeof(*r->vlor_keys), "unsorted keys lie in vlor_ends");
+      static_assert(sizeof(*r->vlor_vals) == sizeof(*r->vlor_keys), "unsorted keys lie in vlor_vals");
       const size_t tb = vlor_sort_temp_bytes(nevents);
       e = cudaMallocAsync(&ev, (size_t)nevents * 2 * sizeof(int32_t), st);
       if (e == cudaSuccess) e = cudaMallocAsync(&temp, tb ? tb : 16, st);
       if (e == cudaSuccess) e = cudaMemcpyAsync(ev, h_events, (size_t)nevents * 2 * sizeof(int32_t), cudaMemcpyHostToDevice, st);
       if (e == cudaSuccess)
-        e = launch_vlor_sort(c->dg, ev, nevents, reinterpret_cast<unsigned long long*>(r->vlor_ends), r->vlor_keys, temp, tb, st);
+        e = launch_vlor_sort(c->dg, ev, nevents, reinterpret_cast<unsigned long long*>(r->vlor_vals), r->vlor_keys, temp, tb, st);
     }
     if (e == cudaSuccess) e = cudaMemsetAsync(r->datos_v, 0, pl.ndata * sizeof(float), st);
     if (e == cudaSuccess) e = launch_vlor_count(c->dg, ev, nevents, r->datos_v, st);
+    if (e == cudaSuccess && nevents > 0 && vlor_by_event(c->dg))
+      e = cudaMemcpyAsync(r->vlor_vals, ev, (size_t)nevents * 2 * sizeof(int32_t), cudaMemcpyDeviceToDevice, st);
     if (ev) cudaFreeAsync(ev, st);
     if (temp) cudaFreeAsync(temp, st);
     if ((s = ck(e, "VLOR events")) != GF_OK) return done(s);

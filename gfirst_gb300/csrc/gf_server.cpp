@@ -277,7 +277,7 @@ gf_status gf_recon_bytes(const gf_geometry* gg, int32_t nsub, const gf_recon_par
     b += 3 * d;                                                                   // staging
   }
   if (p->mode >= 2) b += all * 8 + v;
-  if (p->mode == 3) b += 3 * d + nev * (16 + 16);  // the events' sorted ends, their bins' values
+  if (p->mode == 3) b += 3 * d + nev * (16 + 16);  // the events' sorted ends, gf_recon::vlor_vals
   *bytes = b;
   return GF_OK;
 }

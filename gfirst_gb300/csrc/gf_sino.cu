@@ -423,6 +423,7 @@ cudaError_t launch_blankt(const DevGeom& g, const float* cnt, const float* tsino
 // One 64-bit key per event end, (bin << 32) | (2*event + end), sorted once,
 // puts each bin's shares in that order; the split then sums each bin's run
 // sequentially: the same additions in the same order, without atomics.
+constexpr long long kVlorEventBins = 10 << 20;  // vlor_by_event
 constexpr unsigned long long kNoKey = ~0ull;  // an end of a rejected event
 
 __global__ void vlor_keys_kernel(const int32_t* __restrict__ ev, long long nev, long long ndata,
@@ -453,12 +454,38 @@ cudaError_t launch_vlor_sort(const DevGeom& g, const int32_t* ev, long long nev,
   return cub::DeviceRadixSort::SortKeys(temp, temp_bytes, keys_tmp, keys, (int)(2 * nev), 0, 64, st);
 }
 
-// Both passes walk the sorted ends, so the two file-sized arrays are read in
-// address order; what is random stays in an array of 16 bytes an event.  One
-// pass over the events for their shares, reading projection and weight of two
-// random bins each, and one over the sorted ends for the shares took 61 + 30 us
-// for a million events in 32 M bins; these take 41 + 31.
-// pass 1: projection and weight of each end's bin, ends[2e + end]
+// Two forms.  By event: one pass over the events for both shares of each, which
+// reads projection and weight of two random bins, one over the sorted ends that
+// adds them up.  By end: both passes walk the sorted ends, so the two file-sized
+// arrays are read in address order; what is random stays in an array of 16 bytes an
+// event, and an end's share is worked out where it is added.  By event where both
+// arrays lie in L2.  gf_vlor_split (sort included) of 1 M / 3 M events, by event and
+// by end, us, by the bins: 402, 472 / 989, 1215 at 6 K; 286, 292 / 655, 707 at 0.8 M;
+// 297, 291 / 632, 665 at 7 M; 310, 300 / 653, 668 at 11 M; 319, 306 / 685, 671 at 15 M;
+// 355, 338 / 775, 713 at 32 M; the same within 2 % up to 300 K events.
+bool vlor_by_event(const DevGeom& g) { return (long long)g.P * g.nang * g.nrad <= kVlorEventBins; }
+
+// The share of one end of an event, from projection and weight of its two ends.
+__device__ __forceinline__ float vlor_share(float s1, float s2, float b1, float b2, bool second) {
+  const float valor = __fadd_rn(b1, b2);
+  const float s = __fadd_rn(s1, s2);
+  const float s_inv = (s > 0.01f) ? (float)__drcp_rn((double)s) : 0.f;
+  return __fmul_rn(__fmul_rn(second ? s2 : s1, s_inv), valor);
+}
+
+// by event, pass 1: share[2e + end]
+__global__ void __launch_bounds__(256) vlor_shares_kernel(const int32_t* __restrict__ ev, long long nev, long long ndata,
+                                                          const float* __restrict__ proj, const float* __restrict__ bl,
+                                                          float2* __restrict__ share) {
+  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= nev) return;
+  long long i1, i2;
+  if (!vlor_bins(ev, e, ndata, &i1, &i2)) return;  // its keys are kNoKey: never read
+  const float s1 = proj[i1], s2 = proj[i2], b1 = bl[i1], b2 = bl[i2];
+  share[e] = make_float2(vlor_share(s1, s2, b1, b2, false), vlor_share(s1, s2, b1, b2, true));
+}
+
+// by end, pass 1: projection and weight of each end's bin, ends[2e + end]
 __global__ void __launch_bounds__(256) vlor_ends_kernel(const unsigned long long* __restrict__ keys, long long n,
                                                         const float* __restrict__ proj, const float* __restrict__ bl,
                                                         float2* __restrict__ ends) {
@@ -469,9 +496,11 @@ __global__ void __launch_bounds__(256) vlor_ends_kernel(const unsigned long long
   ends[k & 0xffffffffull] = make_float2(proj[k >> 32], bl[k >> 32]);
 }
 
-// pass 2: the first end of each bin adds the bin's shares in event order
+// pass 2: the first end of each bin adds the bin's shares in event order.  SHARES:
+// vals holds them (by event), else its events' float4 (by end).
+template <bool SHARES>
 __global__ void __launch_bounds__(256) vlor_split_sorted_kernel(const unsigned long long* __restrict__ keys,
-                                                                long long n, const float4* __restrict__ events,
+                                                                long long n, const void* __restrict__ vals,
                                                                 float* out) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -481,11 +510,13 @@ __global__ void __launch_bounds__(256) vlor_split_sorted_kernel(const unsigned l
   if (i > 0 && (keys[i - 1] >> 32) == bin) return;  // not the first share of its bin
   float sum = out[bin];  // the shares are added to out, as the reference adds them to SINOG_VLOR
   for (long long j = i;;) {
-    const float4 e = events[(k & 0xffffffffull) >> 1];  // (projection, weight) of its two ends
-    const float valor = __fadd_rn(e.y, e.w);
-    const float s = __fadd_rn(e.x, e.z);
-    const float s_inv = (s > 0.01f) ? (float)__drcp_rn((double)s) : 0.f;
-    sum = __fadd_rn(sum, __fmul_rn(__fmul_rn((k & 1) ? e.z : e.x, s_inv), valor));
+    const unsigned long long at = k & 0xffffffffull;
+    if (SHARES) {
+      sum = __fadd_rn(sum, static_cast<const float*>(vals)[at]);
+    } else {
+      const float4 e = static_cast<const float4*>(vals)[at >> 1];  // (projection, weight) of its two ends
+      sum = __fadd_rn(sum, vlor_share(e.x, e.z, e.y, e.w, at & 1));
+    }
     if (++j >= n) break;
     k = keys[j];
     if ((k >> 32) != bin) break;
@@ -494,15 +525,22 @@ __global__ void __launch_bounds__(256) vlor_split_sorted_kernel(const unsigned l
 }
 
 cudaError_t launch_vlor_split_sorted(const DevGeom& g, const unsigned long long* keys, long long nev,
-                                     const float* proj, const float* blankt, float2* ends, float* out,
-                                     cudaStream_t st) {
+                                     const int32_t* ev, const float* proj, const float* blankt, float2* vals,
+                                     float* out, cudaStream_t st) {
   if (nev <= 0) return cudaSuccess;
   const long long n = 2 * nev;
   const unsigned nb = (unsigned)((n + 255) / 256);
-  vlor_ends_kernel<<<nb, 256, 0, st>>>(keys, n, proj, blankt, ends);
+  if (vlor_by_event(g))
+    vlor_shares_kernel<<<(unsigned)((nev + 255) / 256), 256, 0, st>>>(ev, nev, (long long)g.P * g.nang * g.nrad, proj,
+                                                                      blankt, vals);
+  else
+    vlor_ends_kernel<<<nb, 256, 0, st>>>(keys, n, proj, blankt, vals);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  vlor_split_sorted_kernel<<<nb, 256, 0, st>>>(keys, n, reinterpret_cast<const float4*>(ends), out);
+  if (vlor_by_event(g))
+    vlor_split_sorted_kernel<true><<<nb, 256, 0, st>>>(keys, n, vals, out);
+  else
+    vlor_split_sorted_kernel<false><<<nb, 256, 0, st>>>(keys, n, vals, out);
   return cudaGetLastError();
 }
 
