@@ -368,7 +368,9 @@ __device__ __forceinline__ float ex2(float x) {
 }
 
 // ---- joint bilateral filter, GFIRST_GPU_Kernels.cu:508-539 ---------------
-// CTA: 8x8 columns x 32 slices, reference and input staged with a halo of 4;
+// CTA: 8x8 columns x 32 slices, reference and input staged with a halo of R (of 4
+// at every R, gf_bilateral on 64x64x32 voxels took 26 us at R = 0 and 28 at 1, now 20
+// and 24);
 // a thread owns one slice (its lane) of BL_N columns along x, so the BL_N + 2 R
 // values of a window row are loaded once for all of them.  Voxels with a
 // coordinate below R give 0 (the reference's unsigned window start wraps and
@@ -389,9 +391,10 @@ __device__ __forceinline__ float ex2(float x) {
 // 128x128x159 voxels takes 449 us with its three layout kernels; one column a
 // thread, with a table lookup, five multiplications and two shared loads a tap,
 // took 1644.
-constexpr int BL_T = 8, BL_H = 4, BL_N = 4;
-constexpr int BL_W = BL_T + 2 * BL_H, BL_Z = 32 + 2 * BL_H + 1;  // staged columns a side, slices and one of padding
-constexpr size_t kBlSmem = (size_t)2 * BL_W * BL_W * BL_Z * sizeof(float);
+constexpr int BL_T = 8, BL_H = 4, BL_N = 4;  // columns a side, largest R, columns of a thread
+constexpr int bl_w(int r) { return BL_T + 2 * r; }           // staged columns a side
+constexpr int bl_z(int r) { return 32 + 2 * r + (r > 0); }   // staged slices; an odd stride where there is a halo
+constexpr size_t bl_smem(int r) { return (size_t)2 * bl_w(r) * bl_w(r) * bl_z(r) * sizeof(float); }
 
 struct BlTaps {
   float lx[BL_H + 1];  // log2 of the spatial weight at distance 0..BL_H along an axis
@@ -412,19 +415,20 @@ __global__ void __launch_bounds__(512, 2) bilateral_kernel(const DevGeom g, cons
                                                            float root_log2e_ci, const BlTaps taps,
                                                            float* __restrict__ out) {
   if (GENERAL && d_max_ref && bl_ordinary(bl_scale(*d_max_ref, root_log2e_ci))) return;
-  extern __shared__ float bl_smem[];
-  float* Sr = bl_smem;
-  float* Si = bl_smem + BL_W * BL_W * BL_Z;
+  constexpr int BL_W = bl_w(R), BL_Z = bl_z(R);
+  extern __shared__ float bl_stage[];
+  float* Sr = bl_stage;
+  float* Si = bl_stage + BL_W * BL_W * BL_Z;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int x0 = blockIdx.x * BL_T, y0 = blockIdx.y * BL_T, z0 = blockIdx.z * 32;
   const int RES = g.res, NZS = g.nzs, NZP = g.nzp;
   for (int c = wid; c < BL_W * BL_W; c += 16) {
     const int yy = c / BL_W, xx = c - yy * BL_W;
-    const int y = y0 - BL_H + yy, x = x0 - BL_H + xx;
+    const int y = y0 - R + yy, x = x0 - R + xx;
     const bool col = y >= 0 && y < RES && x >= 0 && x < RES;
     const long long o = ((long long)y * RES + x) * NZP;
-    for (int zz = lane; zz < 32 + 2 * BL_H; zz += 32) {
-      const int z = z0 - BL_H + zz;
+    for (int zz = lane; zz < 32 + 2 * R; zz += 32) {
+      const int z = z0 - R + zz;
       const bool ok = col && z >= 0 && z < NZS;
       Sr[c * BL_Z + zz] = ok ? img_ld(ref + (o + z)) : __int_as_float(0x7f800000);
       Si[c * BL_Z + zz] = ok ? img_ld(in + (o + z)) : 0.f;
@@ -437,7 +441,7 @@ __global__ void __launch_bounds__(512, 2) bilateral_kernel(const DevGeom g, cons
   const float max_ref = d_max_ref ? *d_max_ref : max_ref_host;
   const float k = bl_scale(max_ref, root_log2e_ci);
   const float rinv = 1.0f / max_ref;
-  const int at = ((ty + BL_H) * BL_W + tx + BL_H) * BL_Z + lane + BL_H;
+  const int at = ((ty + R) * BL_W + tx + R) * BL_Z + lane + R;
   float ref0[BL_N], norm[BL_N], sum[BL_N];
 #pragma unroll
   for (int n = 0; n < BL_N; n++) {
@@ -490,7 +494,7 @@ static cudaError_t launch_bilateral_g(const DevGeom& g, const void* in, const vo
   cudaError_t e = allow_max_smem(k);
   if (e != cudaSuccess) return e;
   const dim3 grid((g.res + BL_T - 1) / BL_T, (g.res + BL_T - 1) / BL_T, g.nzp / 32);
-  k<<<grid, 512, kBlSmem, st>>>(g, static_cast<const T*>(in), static_cast<const T*>(ref), d_max_ref, max_ref, root, taps,
+  k<<<grid, 512, bl_smem(R), st>>>(g, static_cast<const T*>(in), static_cast<const T*>(ref), d_max_ref, max_ref, root, taps,
                                 out);
   return cudaGetLastError();
 }
