@@ -90,7 +90,7 @@ __device__ __forceinline__ Bins<NB> ldg_bins(const float* p) {
 
 // PAIRS: the ratio output is (ratio, mask) pairs.
 template <int R, int NB, bool RATIO, bool FULL, int STORE, bool PAIRS>
-__global__ void __launch_bounds__(512, R == 9 && NB == 1 ? 2 : 1) fp_kernel(const FpArgs a) {
+__device__ __forceinline__ void project(const FpArgs& a) {
   using V = Bins<NB>;
   constexpr int ZV = NB == 1 ? 4 : 2;  // slices resampled by a thread at a time
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -281,8 +281,27 @@ __global__ void __launch_bounds__(512, R == 9 && NB == 1 ? 2 : 1) fp_kernel(cons
 }
 
 template <int R, int NB, bool RATIO, bool FULL, int STORE, bool PAIRS>
+__global__ void __launch_bounds__(512, R == 9 && NB == 1 ? 2 : 1) fp_kernel(const FpArgs a) {
+  project<R, NB, RATIO, FULL, STORE, PAIRS>(a);
+}
+
+// The same for CTAs of 288 threads and more: at 56 to 60 registers two or three fit
+// an SM, at 40 (16 to 20 bytes spilled) three to five.  One bin, 40 registers over
+// the other: 0.98 at 256 threads with the ratio, 1.01 without, 0.92 to 0.98 above
+// (1.02 at 480 without), 1.01 to 1.15 below 224.
+template <int R>
+constexpr int fp_wide_regs = 40;
+
+template <int R, bool RATIO, bool FULL, int STORE, bool PAIRS>
+__global__ void __launch_bounds__(512) __maxnreg__(fp_wide_regs<R>) fp_wide_kernel(const FpArgs a) {
+  project<R, 1, RATIO, FULL, STORE, PAIRS>(a);
+}
+
+template <int R, int NB, bool RATIO, bool FULL, int STORE, bool PAIRS>
 static cudaError_t launch_fp_n(FpArgs a, const FpSchedule& s, int na, cudaStream_t st) {
   auto k = fp_kernel<R, NB, RATIO, FULL, STORE, PAIRS>;
+  if constexpr (R == 9 && NB == 1)
+    if (s.nthreads >= 288) k = fp_wide_kernel<R, RATIO, FULL, STORE, PAIRS>;
   if (NB > 1) a.lc = (s.lc + 1) / 2;  // as many bytes as one bin's steps twice: 43 KB at the default 32 steps and 168 floats a column
   size_t smem = (size_t)a.lc * a.cw * sizeof(Bins<NB>) + (size_t)a.lc * NB * (sizeof(int4) + sizeof(float2));
   if (RATIO) smem = std::max(smem, (size_t)a.g.P * sizeof(float));
