@@ -121,25 +121,26 @@ bool make_fp_schedule(const Plan& p, int R, int lc, FpSchedule* out) {
 // packed arithmetic, but make a quarter of the CTAs with twice the registers:
 // they pay where those fill the GPU and a quarter warp's threads are of one
 // segment.  Four bins' time over one bin's, calls of one context (layout kernel
-// included), at 320 sizes, by the threads of the one-bin grid and of a CTA (nt):
+// included), at 410 sizes, by the threads of the one-bin grid and of a CTA (nt):
 //  - below 150 K threads: 0.81 to 1.61, mean 1.20 (64x64x32, 16 angles: 37 / 27 us);
 //  - nt up to 64: 0.67 to 1.29, mean 0.90;
 //  - nt of 96 to 192 and at least six runs of planes a segment: 0.79 to 1.16, mean
 //    0.95 (15 segments, 21 angles: 201 / 228 us, 168 angles: 1263 / 1641); with
 //    fewer runs 0.82 to 1.20, mean 1.03;
-//  - nt of 224 and 256, two CTAs an SM: below 500 K threads 0.83 to 1.20, mean 0.99,
-//    above 0.80 to 1.01, mean 0.91 (with fewer runs 1.06);
+//  - nt of 224 and 256, two CTAs an SM: below 230 K threads 1.04 to 1.13, above 0.80
+//    to 1.17, mean 0.92 (with fewer runs 1.06);
 //  - nt of 288 to 384, one CTA of 9 to 12 warps an SM: 0.84 to 1.30, mean 1.06;
-//  - nt from 416, one CTA of 13 to 16 warps: below 500 K 1.09 to 1.35, above 0.93 to
-//    1.02 (128x128x159, 53 segments, 10 angles: 273 / 273 us, 320 CTAs on 152 SMs;
-//    190 / 247 a call where another context's kernel fills the last wave).
+//  - nt from 416, one CTA of 13 to 16 warps: below 600 K threads 0.82 to 1.43, mean
+//    1.13, above 0.82 to 1.10, mean 0.96 (128x128x159, 53 segments, 10 angles: 273 /
+//    273 us, 320 CTAs on 152 SMs; 190 / 247 a call where another context's kernel
+//    fills the last wave).
 // With the ratio, whose data the fewer warps wait for, it was 0.82 to 1.52, mean
 // 1.03, at 110 sizes of 1.2 M to 7 M threads, and 1.06 at eight frames of 96^3 in one
 // launch: one bin.
 int fp_bins(const FpSchedule& s, int nseg, int nrad, int views) {
   const int nt = s.nthreads;
   const long long threads = (long long)nrad * views * nt;
-  const bool pays = threads >= (nt < 224 ? 150000 : 500000) && (nt <= 256 || nt >= 416) &&
+  const bool pays = threads >= (nt < 224 ? 150000 : nt <= 256 ? 230000 : 600000) && (nt <= 256 || nt >= 416) &&
                     (nt <= 64 || (int)s.runs.size() >= 6 * nseg);
   const size_t smem = (size_t)((s.lc + 1) / 2) * (s.cw + 6) * 4 * sizeof(float);  // columns, offsets and weights
   return s.R == 9 && pays && smem <= 200 * 1024 ? 4 : 1;

@@ -23,9 +23,10 @@ GEOS = [  # bins a CTA, geometry
     (4, (20, 100, 66, 30, 1, 9, 0.4, 32.0, 16.0)),    # four warps, long runs
     (1, (20, 46, 110, 30, 1, 19, 0.4, 32.0, 16.0)),   # three warps, short segments
     (4, (16, 112, 47, 44, 1, 21, 0.4, 32.0, 12.8)),   # eight warps
-    (1, (16, 112, 47, 40, 1, 21, 0.4, 32.0, 12.8)),   # eight warps, too few threads
+    (1, (16, 112, 47, 18, 1, 21, 0.4, 32.0, 12.8)),   # eight warps, too few threads
     (1, (16, 118, 47, 60, 1, 25, 0.4, 32.0, 12.8)),   # ten warps
     (4, (16, 150, 46, 30, 1, 31, 0.4, 32.0, 12.8)),   # fifteen warps
+    (1, (16, 150, 46, 26, 1, 31, 0.4, 32.0, 12.8)),   # fifteen warps, too few threads
 ]
 
 
