@@ -383,7 +383,7 @@ __device__ __forceinline__ float ex2(float x) {
 // Past the far sides the staged reference is infinite, which makes the weight 0
 // where the intensity scale is a normal number (bl_ordinary).  Other scales -- no
 // range term (an infinite sigmai or max_ref), a product of two ordinary factors
-// that under- or overflows, 0, NaN -- take the GENERAL kernel: the two factors one
+// that under- or overflows, 0, NaN -- take the GENERAL form: the two factors one
 // after the other, taps past the far sides left out by their coordinates.
 //
 // Bound: the 729 exponentials a voxel (16 a clock and SM: 377 us for 128x128x159
@@ -406,15 +406,10 @@ __host__ __device__ __forceinline__ float bl_scale(float max_ref, float root_log
 }
 __host__ __device__ __forceinline__ bool bl_ordinary(float k) { return fabsf(k) >= FLT_MIN && fabsf(k) <= FLT_MAX; }
 
-// With max_ref on the device the GENERAL kernel follows the other one and ends at
-// once where the scale is ordinary (as a test in one kernel it cost 2 %).
 template <class T, int R, bool GENERAL>
-__global__ void __launch_bounds__(512, 2) bilateral_kernel(const DevGeom g, const T* __restrict__ in,
-                                                           const T* __restrict__ ref,
-                                                           const float* __restrict__ d_max_ref, float max_ref_host,
-                                                           float root_log2e_ci, const BlTaps taps,
-                                                           float* __restrict__ out) {
-  if (GENERAL && d_max_ref && bl_ordinary(bl_scale(*d_max_ref, root_log2e_ci))) return;
+__device__ __forceinline__ void bl_filter(const DevGeom& g, const T* __restrict__ in, const T* __restrict__ ref,
+                                          const float* __restrict__ d_max_ref, float max_ref_host, float root_log2e_ci,
+                                          const BlTaps& taps, float* __restrict__ out) {
   constexpr int BL_W = bl_w(R), BL_Z = bl_z(R);
   extern __shared__ float bl_stage[];
   float* Sr = bl_stage;
@@ -487,10 +482,33 @@ __global__ void __launch_bounds__(512, 2) bilateral_kernel(const DevGeom g, cons
   }
 }
 
-template <class T, int R, bool GENERAL>
+// out of line: beside the other form in one function it cost that one 2 %
+template <class T, int R>
+__device__ __noinline__ void bl_filter_general(const DevGeom& g, const T* in, const T* ref, const float* d_max_ref,
+                                               float max_ref_host, float root_log2e_ci, const BlTaps& taps, float* out) {
+  bl_filter<T, R, true>(g, in, ref, d_max_ref, max_ref_host, root_log2e_ci, taps, out);
+}
+
+enum BlForm { kBlOrdinary, kBlGeneral, kBlOnDevice };  // the last: told from a max_ref that only the device knows
+
+template <class T, int R, BlForm FORM>
+__global__ void __launch_bounds__(512, 2) bilateral_kernel(const DevGeom g, const T* __restrict__ in,
+                                                           const T* __restrict__ ref,
+                                                           const float* __restrict__ d_max_ref, float max_ref_host,
+                                                           float root_log2e_ci, const BlTaps taps,
+                                                           float* __restrict__ out) {
+  if constexpr (FORM == kBlOnDevice)
+    if (!bl_ordinary(bl_scale(*d_max_ref, root_log2e_ci))) {
+      bl_filter_general<T, R>(g, in, ref, d_max_ref, max_ref_host, root_log2e_ci, taps, out);
+      return;
+    }
+  bl_filter<T, R, FORM == kBlGeneral>(g, in, ref, d_max_ref, max_ref_host, root_log2e_ci, taps, out);
+}
+
+template <class T, int R, BlForm FORM>
 static cudaError_t launch_bilateral_g(const DevGeom& g, const void* in, const void* ref, const float* d_max_ref,
                                       float max_ref, float root, const BlTaps& taps, float* out, cudaStream_t st) {
-  auto k = bilateral_kernel<T, R, GENERAL>;
+  auto k = bilateral_kernel<T, R, FORM>;
   cudaError_t e = allow_max_smem(k);
   if (e != cudaSuccess) return e;
   const dim3 grid((g.res + BL_T - 1) / BL_T, (g.res + BL_T - 1) / BL_T, g.nzp / 32);
@@ -502,13 +520,10 @@ static cudaError_t launch_bilateral_g(const DevGeom& g, const void* in, const vo
 template <class T, int R>
 static cudaError_t launch_bilateral_r(const DevGeom& g, const void* in, const void* ref, const float* d_max_ref,
                                       float max_ref, float root, const BlTaps& taps, float* out, cudaStream_t st) {
-  const bool ordinary = bl_ordinary(bl_scale(max_ref, root));  // of a max_ref known here
-  cudaError_t e = cudaSuccess;
-  if (d_max_ref || ordinary)
-    e = launch_bilateral_g<T, R, false>(g, in, ref, d_max_ref, max_ref, root, taps, out, st);
-  if (e == cudaSuccess && (d_max_ref || !ordinary))
-    e = launch_bilateral_g<T, R, true>(g, in, ref, d_max_ref, max_ref, root, taps, out, st);
-  return e;
+  if (d_max_ref) return launch_bilateral_g<T, R, kBlOnDevice>(g, in, ref, d_max_ref, max_ref, root, taps, out, st);
+  if (bl_ordinary(bl_scale(max_ref, root)))
+    return launch_bilateral_g<T, R, kBlOrdinary>(g, in, ref, nullptr, max_ref, root, taps, out, st);
+  return launch_bilateral_g<T, R, kBlGeneral>(g, in, ref, nullptr, max_ref, root, taps, out, st);
 }
 
 template <class T>
