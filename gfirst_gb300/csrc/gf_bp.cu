@@ -8,7 +8,7 @@
 // Two kernels compute the same sums with the same operations in the same
 // order: this one, and the column tiles of gf_bp_tile.cu, which take 60 % of the
 // instructions and 40 % of the shared-memory wavefronts a voxel but need
-// more columns to fill the GPU.  Small images run this one (bp_uses_tiles in
+// more columns to fill the GPU.  Small images run this one (tiles_pay in
 // gf_plan.cpp has the line and the times of both sides), and so do geometries
 // whose tiles do not fit shared memory and masks with other values than 1 and
 // -1000 (gf_back_project only).

@@ -27,10 +27,10 @@
 // segments whose runs share a warp (NB = 1: 2.06 wavefronts per load; NB = 4,
 // where a load is served by quarter warps: 1.4).  128x128x159 voxels, 53
 // segments, 10 angles with the ratio 268 -> 250 us by resampling four slices a
-// thread and reading the data in whole lines; 15 segments, 21 angles 279 ->
-// 221; the whole sinogram of 168 angles x 1293 planes 1933 -> 1292 (four bins);
-// 64x64x32 voxels, 16 angles 36 -> 29.  Two bins a CTA (264, 222 with the
-// ratio) lost to either side of it.
+// thread and reading the data in whole lines, 241 with 40 registers; 15 segments,
+// 21 angles 279 -> 221; the whole sinogram of 168 angles x 1293 planes 1934 -> 1263
+// (four bins); 64x64x32 voxels, 16 angles 36 -> 29.  Two bins a CTA (264, 222 with
+// the ratio) lost to either side of it.
 #include <algorithm>
 
 #include "gf_kernels.h"
