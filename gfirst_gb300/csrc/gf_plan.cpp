@@ -239,7 +239,10 @@ static long long run_ctas(const Plan& p) {
 // 1.13 at 98 x 98 x 86 and 31.  It leaves to columns a few that gain without masked
 // bins (97 x 97 x 117: 0.93; 98 x 98 x 86: 0.80), and the first one more (90 x 90 x
 // 54, 29 segments: 0.73, 0.97 with; 115 x 115 x 51, 5: 0.76, 0.95), because their
-// neighbours lose as much with them (84 x 84 x 54, 15: 1.24 per voxel).
+// neighbours lose as much with them (84 x 84 x 54, 15: 1.24 per voxel).  Masks of
+// whole bins, planes or diagonal gaps cost less than 2 % at random (96^3: 0.78 to 0.83
+// per view, 0.88 to 0.93 per voxel), 10 to 50 % at random more: up to 1.03 and 1.19
+// at 96^3, 0.87 and 0.92 at 128 x 128 x 159.
 static bool tiles_pay(const Plan& p) {
   const BpTile t = tile_shape(p, 8, 4, kTileRun);  // the largest of its slots
   if (2ll * t.warps * t.slot_bytes + 32ll * p.amax > 160 * 1024) return false;
